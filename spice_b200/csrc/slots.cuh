@@ -419,7 +419,9 @@ __device__ __forceinline__ void window_slots_body( net_params const & p, int con
 						long long const need = t0 + k + 4 - p.delay;
 						if( k + 4 < L && need >= 0 && need > s_known )
 						{
-							long long const demand = min( t0 + k - P - 1, need + 7 );
+							// no further than the last step this launch reads: in a window (L <= delay),
+							// whose CTAs need not be resident at once, that is before the launch
+							long long const demand = min( min( t0 + k - P - 1, need + 7 ), t0 + L - 1 - p.delay );
 							warp_wait_all_published( p, demand );
 							if( lane == 0 ) s_known = demand;
 						}
