@@ -23,7 +23,7 @@ ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libspice_b200.so")
 SOURCES = [os.path.join(HERE, "csrc", "net.cu"), os.path.join(HERE, "csrc", "server.cpp")]
 DEPS = SOURCES + [os.path.join(HERE, "csrc", f) for f in
-                  ("kernels.cuh", "plastic.cuh", "flat.cuh", "slots.cuh", "ordered.cuh", "models.cuh", "device_common.cuh")]
+                  ("kernels.cuh", "plastic.cuh", "flat.cuh", "dense.cuh", "slots.cuh", "ordered.cuh", "models.cuh", "device_common.cuh")]
 USER_MODEL_ID = 7
 
 

@@ -1,0 +1,872 @@
+// window_dense: the window kernel of nets whose rows are dense enough to be target bitmaps.
+//
+// Same results as window_flat (flat.cuh). Instead of index lists a source's row is one bit
+// per target, cut by destination tile: bits[src][unit of tile j ...], 64 targets to a unit,
+// a tile's units padded to whole 32-byte sectors. At the usual densities (p = 0.1) a row's
+// part in a tile of 512 neurons is 64 bytes against 80 bytes of 10-bit indices plus a
+// record, its place follows from the source's id alone, and, above all, arrivals are
+// counted 64 targets at a time: a carry-save adder over seven rows costs sixteen logic
+// operations per 64 targets where index lists cost a shared-memory atomic per synapse.
+//
+// Besides the spike ring every step has one list of its spikes over all tiles, class 0 from
+// the front and class 1 from the back, which the tiles' publishers append to (the order
+// within a class does not matter to counts). No fence is needed on the way: a step's word
+// (step_word) counts the tiles that have added theirs, and their spikes of both classes, in
+// one 64-bit atomic addition per tile, which also returns the tile's place; and every list
+// entry carries its step (plus one: fresh memory is no entry), so a reader sees whether it has arrived. (With a fence and a
+// flag per tile, a publication took as long as the count warps kept loading rows: the fence
+// waits for the whole SM's loads. 28,000 cycles a round at 1e8 synapses.) The words are
+// never reset: a step's numbers are its word less the word's value before the step.
+//
+// A CTA owns a tile of neurons with inputs and a tile without (Brunel's Poisson sources), so
+// the sources' random numbers fill the issue slots that waiting for rows leaves free.
+//
+// Steps run in rounds of `m` (up to DN_MB) steps. A spike reaches its targets `delay` steps
+// later, so with 3 m <= delay the spikes that the next two rounds read are fired before
+// this round begins, and a CTA works on four rounds at once, in ticks of one block barrier.
+// A tick's work is cut into items that the warps take from a queue, the longest first:
+//   - publishing (r - 1), an item per step: the spikes to the ring and the step's list;
+//   - counting (r + 1): an item sums the bitmap rows of one step's arrivals of one class (class
+//     0 in two halves) in 256 columns, to one byte per target;
+//   - scouting (r + 2), an item per step: waits until every tile has added its spikes of the
+//     source step, and fetches their ids;
+//   - updating (r), an item per 32 neurons: replays the counts through the model's receive()
+//     and runs update(), one thread per neuron through all of the round's steps.
+// Shorter delays and launches of one or two steps run the same items stage by stage.
+//
+// Measured (us per step, window_flat before, this kernel after): Brunel 1e9 6.55 -> 3.49, 4e8
+// 4.32 -> 2.58, 1e8 3.99 -> 1.40, 1e7 3.16 -> 1.12 (delay 15); 1e8 at delay 7 3.89 -> 2.63,
+// at delay 1 11.2 -> 8.5; VA 1e8 (p = 0.02, delay 8) 4.01 -> 2.18. Bound by instruction issue:
+// 48 % of issue slots at 3.2e8 synapses, the logic pipe at 38 %, shared-memory round trips
+// the leading stall; with every row read from L2 (the same row over and over) 1e9 takes
+// 2.88 instead of 3.49.
+// Why a queue: a stage is a chain of dependent instructions (about one in 12 cycles a warp),
+// so a tick is short only if all warps are busy all along; with fixed roles the slowest
+// role's few warps set its length (at 1e9 synapses 40,000 cycles of updates in 8 warps).
+#pragma once
+
+#include "flat.cuh"
+
+namespace spk
+{
+// 85 registers a thread: at 1,024 threads the count items spill (Brunel 1e9 3.60 us per step,
+// 1e8 1.50), at 512 too few warps hide latency (3.68, 1.55); 768: 3.46, 1.40
+constexpr int DN_THREADS = 768;
+constexpr int DN_MB = 5;        // steps of a round at most
+constexpr int DN_LIST = 8192;   // a round's ids kept in shared memory
+constexpr int DN_SUM = 8;       // bit planes of a lane's own sums (at most 255 rows)
+constexpr int DN_OUT = 16;      // bit planes of an item's sums: a target's in-degree must be less
+constexpr int DN_MAX_IN = ( 1 << DN_OUT ) - 1;
+constexpr int DN_CHUNK = 4;     // units a count item takes: four lanes a row, eight rows a load
+constexpr int DN_ROWS = 56;     // rows of a turn of its loop
+constexpr int DN_MAX_TILE = 1536;
+constexpr int DN_CLASSES = 2;   // a step's list holds two classes, from its two ends
+constexpr size_t DN_CTX_BYTES = 2048;
+// parts of a step's arrivals: class 0 in two halves, class 1
+__host__ __device__ constexpr int dense_parts( int classes ) { return classes + 1; }
+
+// 64-target units of a tile of `span` neurons, whole 32-byte sectors
+__host__ __device__ inline int dense_units( int span ) { return ( span + 255 ) / 256 * 4; }
+
+// Steps the step lists hold. A tile that writes step t has seen step t - delay complete: every
+// tile has added its spikes of that step, so every one has read the lists up to step
+// t - 2 delay, and knows the final word of step t - 3 delay, whose place step t takes.
+__host__ __device__ inline int dense_ring( int delay ) { return 3 * delay; }
+
+// shared memory of a CTA: the working set (dense_ctx), for both its tiles neuron state
+// [attrs][span] and fired bits [2][m][words], the steps' words before their steps [ring], and,
+// if it has a tile with inputs, counts [2][m][parts][low bytes, high bytes][columns], the
+// rounds' ids [2][DN_LIST] and every warp's ids of a step that is not among them
+struct dense_geom
+{
+	int words[2];
+	size_t state[2], bits[2], words_before, counts, ids, own, end;
+};
+__host__ __device__ inline dense_geom dense_layout( int classes, int attrs, int span_in, int span_free, int m, int delay )
+{
+	dense_geom g;
+	int const span[2] = { span_in, span_free };
+	auto up = []( size_t b ) { return ( b + 15 ) & ~(size_t)15; };
+	size_t o = DN_CTX_BYTES;
+	for( int i = 0; i < 2; i++ )
+	{
+		g.words[i] = ( span[i] + 31 ) / 32;
+		g.state[i] = o;
+		g.bits[i] = up( o + (size_t)attrs * span[i] * 4 );
+		o = up( g.bits[i] + (size_t)2 * m * g.words[i] * 4 );
+	}
+	g.words_before = o;
+	g.counts = up( g.words_before + (size_t)dense_ring( delay ) * 8 );
+	g.end = g.own = g.ids = g.counts;
+	if( span_in == 0 ) return g;
+	g.ids = up( g.counts + (size_t)2 * m * dense_parts( classes ) * 2 * ( ( span_in + 255 ) / 256 * 256 ) );
+	g.own = g.ids + (size_t)2 * DN_LIST * 4;
+	g.end = g.own + (size_t)( DN_THREADS / 32 ) * DN_ROWS * 4;
+	return g;
+}
+// steps of a round for a net's delay: three rounds in flight within it
+__host__ __device__ inline int dense_round( int delay )
+{
+	int const m = delay < 3 ? delay : delay / 3;
+	return m > DN_MB ? DN_MB : m;
+}
+__device__ __forceinline__ unsigned long long dense_word( int zeros, int ones ) { return 1ull << 48 | (unsigned long long)ones << 24 | (unsigned long long)zeros; }
+constexpr int DN_MAX_N = 1 << 24; // spikes of a class fit a word's 24 bits, tiles its 16
+
+// ------------------------------------------------------------------------------------
+// building the bitmaps (once per net)
+// ------------------------------------------------------------------------------------
+// tile_inputs[tile] <- 1 if any row has synapses in the tile
+__global__ void __launch_bounds__( 256 ) dense_tile_inputs( int n, int ntiles, unsigned const * pivots, int * tile_inputs )
+{
+	int const nw = ( gridDim.x * blockDim.x ) >> 5, lane = threadIdx.x & 31;
+	for( int src = ( blockIdx.x * blockDim.x + threadIdx.x ) >> 5; src < n; src += nw )
+	{
+		unsigned const * pv = pivots + (long long)src * ( ntiles + 1 );
+		for( int j = lane; j < ntiles; j += 32 )
+			if( pv[j + 1] > pv[j] && !*(int volatile *)( tile_inputs + j ) ) atomicOr( tile_inputs + j, 1 );
+	}
+}
+
+// the bit of target d within a row: its tile's first unit and its place in the tile
+__global__ void __launch_bounds__( 256 ) dense_positions( int n, int ntiles, int const * tile_first, int const * tile_unit, int * bitpos )
+{
+	int const d = blockIdx.x * blockDim.x + threadIdx.x;
+	if( d >= n ) return;
+	int lo = 0, hi = ntiles;
+	while( hi - lo > 1 )
+	{
+		int const mid = ( lo + hi ) >> 1;
+		if( tile_first[mid] <= d )
+			lo = mid;
+		else
+			hi = mid;
+	}
+	bitpos[d] = tile_unit[lo] * 64 + ( d - tile_first[lo] );
+}
+
+// One CTA per row at a time: the row's bits set in shared memory, then written out; chunk c of
+// a row (four units) of source src goes to unit chunks[c].x + src * chunks[c].y.
+__global__ void __launch_bounds__( 512 ) dense_fill(
+    int n, int width, int row_units, int const * edges, int const * bitpos, longlong2 const * chunks, uint2 * bits )
+{
+	extern __shared__ __align__( 16 ) unsigned row_bits[];
+	for( int src = blockIdx.x; src < n; src += gridDim.x )
+	{
+		for( int x = threadIdx.x; x < 2 * row_units; x += blockDim.x ) row_bits[x] = 0u;
+		__syncthreads();
+		int4 const * row = reinterpret_cast<int4 const *>( edges + (long long)src * width ); // width is a multiple of 32
+		for( int x = threadIdx.x; x < width / 4; x += blockDim.x )
+		{
+			int4 const d = __ldcs( row + x );
+			int const e[4] = { d.x, d.y, d.z, d.w };
+#pragma unroll
+			for( int i = 0; i < 4; i++ )
+				if( (unsigned)e[i] < (unsigned)n )
+				{
+					int const b = __ldg( bitpos + e[i] );
+					atomicOr( row_bits + ( b >> 5 ), 1u << ( b & 31 ) );
+				}
+		}
+		__syncthreads();
+		for( int x = threadIdx.x; x < row_units / 2; x += blockDim.x )
+		{
+			longlong2 const c = __ldg( chunks + ( x >> 1 ) );
+			reinterpret_cast<uint4 *>( bits + c.x + src * c.y )[x & 1] = reinterpret_cast<uint4 const *>( row_bits )[x];
+		}
+		__syncthreads();
+	}
+}
+
+// ------------------------------------------------------------------------------------
+// step lists
+// ------------------------------------------------------------------------------------
+// The lists of the `delay` steps before `now` from the spike ring (a restored net), one CTA
+// per step; the lists are empty before.
+template <typename Model>
+__global__ void __launch_bounds__( 256 ) dense_lists_from_ring( net_params p, long long now )
+{
+	using N = typename Model::neuron;
+	snn_info const info{ p.n };
+	long long const t = now - 1 - blockIdx.x;
+	if( t < 0 ) return;
+	long long const slot = t % p.ring;
+	int const ls = (int)( t % dense_ring( p.delay ) );
+	unsigned long long * list = p.step_ids + (long long)ls * p.n;
+	for( int i = threadIdx.x; i < p.ntiles; i += blockDim.x )
+	{
+		int const c = (int)p.ring_cnt[slot * p.ntiles + i];
+		int const * ids = p.ring_ids + slot * p.n + p.tile_first[i];
+		int ones = 0;
+		for( int a = 0; a < c; a++ ) ones += N::input_class( ids[a], info );
+		unsigned long long const at = atomicAdd( p.step_word + ls, dense_word( c - ones, ones ) );
+		int o0 = (int)( at & 0xFFFFFF ), o1 = p.n - 1 - (int)( at >> 24 & 0xFFFFFF );
+		for( int a = 0; a < c; a++ )
+			list[N::input_class( ids[a], info ) ? o1-- : o0++] = (unsigned long long)(unsigned)( t + 1 ) << 32 | (unsigned)ids[a];
+	}
+}
+
+// ------------------------------------------------------------------------------------
+// window kernel
+// ------------------------------------------------------------------------------------
+// full adder over 32 independent bits: sum and carry of a + b + c
+__device__ __forceinline__ unsigned maj3( unsigned a, unsigned b, unsigned c ) { return ( a & b ) | ( c & ( a ^ b ) ); }
+__device__ __forceinline__ void full_add( unsigned & a, unsigned b, unsigned & c )
+{
+	unsigned const s = a ^ b ^ c;
+	c = maj3( a, b, c );
+	a = s;
+}
+__device__ __forceinline__ unsigned long long load_relaxed( unsigned long long const * q )
+{
+	unsigned long long v;
+	asm volatile( "ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"( v ) : "l"( q ) : "memory" );
+	return v;
+}
+__device__ __forceinline__ void store_relaxed( unsigned long long * q, unsigned long long v ) { asm volatile( "st.relaxed.gpu.global.u64 [%0], %1;" ::"l"( q ), "l"( v ) : "memory" ); }
+// a row is read once per step it arrives in: past L1
+__device__ __forceinline__ uint2 load_row( uint2 const * q )
+{
+	uint2 v;
+	asm volatile( "ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"( v.x ), "=r"( v.y ) : "l"( q ) );
+	return v;
+}
+
+// A CTA's working set: the net, the launch and the tile, at the start of its shared memory
+// (the arrays after it as byte offsets, so that every access is a shared-memory one). The
+// items are functions of their own (not inlined): each gets the whole register budget, where
+// one body with all of them kept the others' values alive and spilled.
+struct dense_ctx
+{
+	net_params p;
+	int cta, L, m, list_ring, last;
+	int tile[2], d0[2], span[2], words[2]; // the tile with inputs and the one without (span 0: none)
+	int units, chunks, cols, cap;          // of the tile with inputs; ids a step's list holds
+	int slot0, list0;      // ring slot and list of step t0
+	longlong2 place;       // the tile's first unit in the bitmaps, and units from row to row
+	long long t0;          // first step of the launch
+	float c, sum, dt;      // the simulated clock
+	// byte offsets
+	int state[2];
+	int bits[2];      // [2][m][words] fired bits
+	int words_before; // [list_ring] every list's word before its step (64 bits)
+	int counts;       // [2][m][parts][2][cols]
+	int ids;          // [2][m][cap]
+	int own;          // [warps][DN_ROWS]
+	unsigned queue[4];                // items taken of tick t at t & 3
+	float dts[MAX_WINDOW];            // dt of step k at k % MAX_WINDOW
+	int n[4][DN_MB][DN_CLASSES];      // arrivals of round r at r & 3
+	int high[4][DN_MB];               // some count of the step needs its high byte
+
+	__device__ __forceinline__ int steps( int r ) const { return min( L - r * m, m ); }
+	// ring slot and list of the step k steps into the launch, k >= -delay
+	__device__ __forceinline__ int slot( int k ) const { return (int)( (unsigned)( slot0 + k + p.ring ) % (unsigned)p.ring ); }
+	__device__ __forceinline__ int list( int k ) const { return (int)( (unsigned)( list0 + k + list_ring ) % (unsigned)list_ring ); }
+	// by one thread, round by round: the dt of round r's steps
+	__device__ __forceinline__ void advance_clock( int r )
+	{
+		for( int k = r * m; k < min( L, ( r + 1 ) * m ); k++ )
+		{
+			float const d = kahan_add( c, sum, dt );
+			dts[k % MAX_WINDOW] = d;
+			if( cta == 0 ) p.dt_ring[( t0 + k ) % DT_RING] = d;
+		}
+	}
+};
+static_assert( sizeof( dense_ctx ) <= DN_CTX_BYTES, "the working set's place" );
+extern __shared__ __align__( 128 ) unsigned char dense_smem[];
+template <typename T>
+__device__ __forceinline__ T * dense_at( int offset )
+{
+	return reinterpret_cast<T *>( dense_smem + offset );
+}
+__device__ __forceinline__ dense_ctx & dense_get() { return *dense_at<dense_ctx>( 0 ); }
+
+// Waits, by one warp, until every tile has added its spikes of the step k steps into the
+// launch; returns their numbers (zeros | ones << 24; nothing before step 0), and the word
+// becomes the one before the next step that takes the list's place. A wait that runs out
+// sets ERR_TIMEOUT and returns.
+__device__ __forceinline__ unsigned long long dense_wait( int k )
+{
+	dense_ctx & x = dense_get();
+	if( x.t0 + k < 0 ) return 0;
+	int const l = x.list( k );
+	unsigned long long & before = dense_at<unsigned long long>( x.words_before )[l];
+	unsigned long long const was = before;
+	unsigned long long got = 0;
+	for( int it = 0;; it++ )
+	{
+		got = load_relaxed( x.p.step_word + l ) - was;
+		if( __all_sync( 0xffffffffu, (int)( got >> 48 ) == x.p.ntiles ) ) break;
+		if( it >= x.p.wait_limit || ( *(int volatile *)x.p.err & ERR_TIMEOUT ) )
+		{
+			atomicOr( x.p.err, ERR_TIMEOUT );
+			break;
+		}
+		__nanosleep( 64 );
+	}
+	got = __shfl_sync( 0xffffffffu, got, 0 );
+	if( ( threadIdx.x & 31 ) == 0 ) before = was + got;
+	__syncwarp();
+	return got & 0xFFFFFFFFFFFFull;
+}
+
+// Update item, the tile with inputs: the steps of round r for the neurons of word w: counts
+// replayed, update, fired bits. Column j of a word lies at byte 4 (j % 8) + j / 8.
+template <typename Model>
+__device__ __noinline__ void dense_update( int r, int w )
+{
+	dense_ctx & x = dense_get();
+	using N = typename Model::neuron;
+	using Tup = typename N::template apply<reg_tuple>;
+	constexpr int C = N::input_classes, P = dense_parts( C );
+	int const lane = threadIdx.x & 31, span = x.span[0], steps = x.steps( r ), cols = x.cols;
+	snn_info const info{ x.p.n };
+	unsigned long long const seed = x.p.seed;
+	unsigned char const * cb = dense_at<unsigned char const>( x.counts ) + (size_t)( r & 1 ) * x.m * P * 2 * cols + w * 32 + ( lane & 7 ) * 4 + ( lane >> 3 );
+	unsigned * fb = dense_at<unsigned>( x.bits[0] ) + ( r & 1 ) * x.m * x.words[0] + w;
+	unsigned char * state = dense_at<unsigned char>( x.state[0] );
+	int const k0 = r * x.m, local = w * 32 + lane;
+	uint32_t const step0 = (uint32_t)( x.t0 + k0 );
+	bool const mine = local < span;
+	uint32_t const i = (uint32_t)( x.d0[0] + ( mine ? local : 0 ) );
+	Tup st;
+	smem_state<N>::load( st, state, span, mine ? local : 0 );
+	reg_iter<Tup> it{ st, i };
+	for( int s = 0; s < steps; s++, cb += P * 2 * cols, fb += x.words[0] )
+	{
+		unsigned in[2] = { (unsigned)cb[0] + cb[2 * cols], C > 1 ? (unsigned)cb[4 * cols] : 0u };
+		if( x.high[r & 3][s] )
+		{
+			in[0] += ( (unsigned)cb[cols] + cb[3 * cols] ) << 8;
+			if( C > 1 ) in[1] += (unsigned)cb[5 * cols] << 8;
+		}
+		bool fired = false;
+		if( mine )
+		{
+#pragma unroll
+			for( int c = 0; c < C; c++ )
+				if( in[c] )
+				{
+					chain_backend rb( seed, i, step0 + s, in[c] );
+					N::receive( N::class_source( c, info ), it, null_syn_iter{}, info, rb );
+				}
+			device_backend bak( seed, i, step0 + s );
+			fired = N::update( it, x.dts[( k0 + s ) % MAX_WINDOW], info, bak );
+		}
+		unsigned const word = __ballot_sync( 0xffffffffu, fired );
+		if( lane == 0 ) *fb = word;
+	}
+	if( mine ) smem_state<N>::store( st, state, span, local );
+}
+
+// Update item, the tile without inputs. A round's steps of one neuron in one unrolled
+// stretch: the parts of the counter generator that do not depend on the step are computed
+// once.
+template <typename Model>
+__device__ __noinline__ void dense_update_free( int r, int w )
+{
+	dense_ctx & x = dense_get();
+	using N = typename Model::neuron;
+	using Tup = typename N::template apply<reg_tuple>;
+	int const lane = threadIdx.x & 31, W = x.words[1], span = x.span[1], steps = x.steps( r );
+	snn_info const info{ x.p.n };
+	unsigned long long const seed = x.p.seed;
+	unsigned * fb = dense_at<unsigned>( x.bits[1] ) + ( r & 1 ) * x.m * W;
+	unsigned char * state = dense_at<unsigned char>( x.state[1] );
+	int const k0 = r * x.m, local = w * 32 + lane;
+	uint32_t const step0 = (uint32_t)( x.t0 + k0 );
+	bool const mine = local < span;
+	uint32_t const i = (uint32_t)( x.d0[1] + ( mine ? local : 0 ) );
+	Tup st;
+	smem_state<N>::load( st, state, span, mine ? local : 0 );
+	reg_iter<Tup> it{ st, i };
+	auto step = [&]( int s ) {
+		device_backend bak( seed, i, step0 + s );
+		bool const fired = N::update( it, x.dts[( k0 + s ) % MAX_WINDOW], info, bak ) && mine;
+		unsigned const word = __ballot_sync( 0xffffffffu, fired );
+		if( lane == 0 ) fb[s * W + w] = word;
+	};
+	if( steps == DN_MB )
+#pragma unroll
+		for( int s = 0; s < DN_MB; s++ ) step( s );
+	else
+#pragma unroll 1
+		for( int s = 0; s < steps; s++ ) step( s );
+	if( mine ) smem_state<N>::store( st, state, span, local );
+}
+
+// Publishing item, step s of round r: for both tiles the step's spikes, ascending, to
+// the ring (compact_step's order and format), and to the step's list.
+template <typename Model>
+__device__ __noinline__ void dense_publish( int r, int s )
+{
+	dense_ctx & x = dense_get();
+	using N = typename Model::neuron;
+	constexpr int C = N::input_classes;
+	int const lane = threadIdx.x & 31, n = x.p.n, k = r * x.m + s;
+	snn_info const info{ n };
+	long long const row = (long long)x.slot( k );
+	int const l = x.list( k );
+	unsigned long long * const list = x.p.step_ids + (long long)l * n;
+	unsigned long long const tag = (unsigned long long)(unsigned)( x.t0 + k + 1 ) << 32;
+	// spikes by class, then this CTA's place in the list
+	int all[2], one[2];
+#pragma unroll
+	for( int h = 0; h < 2; h++ )
+	{
+		all[h] = one[h] = 0;
+		if( x.span[h] == 0 ) continue;
+		unsigned const * fb = dense_at<unsigned const>( x.bits[h] ) + (size_t)( ( r & 1 ) * x.m + s ) * x.words[h];
+		for( int w = lane; w < x.words[h]; w += 32 )
+		{
+			unsigned f = fb[w];
+			all[h] += __popc( f );
+			if( C > 1 )
+				for( ; f; f &= f - 1 ) one[h] += N::input_class( x.d0[h] + w * 32 + __ffs( f ) - 1, info );
+		}
+		all[h] = __reduce_add_sync( 0xffffffffu, all[h] );
+		if( C > 1 ) one[h] = __reduce_add_sync( 0xffffffffu, one[h] );
+	}
+	unsigned long long at = 0;
+	if( lane == 0 )
+	{
+		unsigned long long add = 0;
+#pragma unroll
+		for( int h = 0; h < 2; h++ )
+			if( x.span[h] )
+			{
+				x.p.ring_cnt[row * x.p.ntiles + x.tile[h]] = (unsigned)all[h];
+				if( x.tile[h] != x.p.withhold_tile ) add += dense_word( all[h] - one[h], one[h] );
+			}
+		at = atomicAdd( x.p.step_word + l, add ) - dense_at<unsigned long long>( x.words_before )[l];
+	}
+	int b0 = __shfl_sync( 0xffffffffu, (int)( at & 0xFFFFFF ), 0 ), b1 = __shfl_sync( 0xffffffffu, (int)( at >> 24 & 0xFFFFFF ), 0 );
+#pragma unroll
+	for( int h = 0; h < 2; h++ )
+	{
+		if( all[h] == 0 ) continue;
+		int const W = x.words[h], d0 = x.d0[h];
+		unsigned const * fb = dense_at<unsigned const>( x.bits[h] ) + (size_t)( ( r & 1 ) * x.m + s ) * W;
+		int * out = x.p.ring_ids + row * n + d0;
+		int done = 0, done1 = 0;
+		for( int w0 = 0; w0 < W; w0 += 32 )
+		{
+			int const w = w0 + lane;
+			unsigned f = w < W ? fb[w] : 0u;
+			if( !__any_sync( 0xffffffffu, f != 0u ) ) continue;
+			int ones = 0;
+			if( C > 1 && one[h] )
+				for( unsigned g = f; g; g &= g - 1 ) ones += N::input_class( d0 + w * 32 + __ffs( g ) - 1, info );
+			int const c = __popc( f );
+			int const incl = warp_inclusive_scan( c ), incl1 = C > 1 && one[h] ? warp_inclusive_scan( ones ) : 0;
+			int off = done + incl - c, off1 = done1 + incl1 - ones;
+			for( ; f; f &= f - 1 )
+			{
+				int const id = d0 + w * 32 + __ffs( f ) - 1;
+				bool const is1 = C > 1 && one[h] && N::input_class( id, info ) != 0;
+				int const o = is1 ? n - 1 - ( b1 + off1 ) : b0 + off - off1;
+				if( (unsigned)o < (unsigned)n ) store_relaxed( list + o, tag | (unsigned)id ); // in range unless a wait ran out
+				out[off++] = id;
+				off1 += is1;
+			}
+			done += __shfl_sync( 0xffffffffu, incl, 31 );
+			done1 += __shfl_sync( 0xffffffffu, incl1, 31 );
+		}
+		b0 += all[h] - one[h];
+		b1 += one[h];
+	}
+}
+
+// The entry of a step's list that holds the o-th spike of class c, and its id once it is
+// there: a counted entry that is not is a store on its way.
+__device__ __forceinline__ unsigned long long const * dense_entry( int k, int c, int o )
+{
+	dense_ctx & x = dense_get();
+	return x.p.step_ids + (long long)x.list( k ) * x.p.n + ( c ? x.p.n - 1 - o : o );
+}
+__device__ __forceinline__ int dense_id( unsigned tag, unsigned long long const * q, unsigned long long v )
+{
+	dense_ctx & x = dense_get();
+	for( int it = 0; (unsigned)( v >> 32 ) != tag; it++ )
+	{
+		if( it >= x.p.wait_limit || ( *(int volatile *)x.p.err & ERR_TIMEOUT ) )
+		{
+			atomicOr( x.p.err, ERR_TIMEOUT );
+			break;
+		}
+		v = load_relaxed( q );
+	}
+	return (int)(unsigned)v;
+}
+
+// Scout item, step s of round r: waits until every tile has added its spikes of the source
+// step and, for a tile with inputs, fetches their ids, if they fit: class 0 from the front of
+// the step's part of the list, class 1 from its back.
+template <int C>
+__device__ __noinline__ void dense_scout( int r, int s )
+{
+	dense_ctx & x = dense_get();
+	int const lane = threadIdx.x & 31, k = r * x.m + s - x.p.delay, cap = x.cap;
+	if( s == 0 && lane == 0 && r > 0 ) x.advance_clock( r );
+	unsigned long long const got = dense_wait( k );
+	// in range unless a wait ran out
+	int const n[2] = { min( (int)( got & 0xFFFFFF ), x.p.n ), C > 1 ? min( (int)( got >> 24 ), x.p.n ) : 0 };
+	if( lane < 2 ) x.n[r & 3][s][lane] = lane ? n[1] : n[0];
+	if( lane == 0 ) x.high[r & 3][s] = 0;
+	if( x.span[0] == 0 || n[0] + n[1] > cap ) return;
+	unsigned const tag = (unsigned)( x.t0 + k + 1 );
+	constexpr int B = 8; // entries in flight per lane
+#pragma unroll 1
+	for( int c = 0; c < C; c++ )
+	{
+		int const dir = c ? -1 : 1, ng = c ? n[1] : n[0];
+		int * list = dense_at<int>( x.ids ) + ( ( r & 1 ) * x.m + s ) * cap + ( c ? cap - 1 : 0 );
+		unsigned long long const * const q = dense_entry( k, c, 0 );
+		for( int o0 = lane; o0 < ng; o0 += 32 * B )
+		{
+			unsigned long long v[B];
+			bool here = true;
+#pragma unroll
+			for( int b = 0; b < B; b++ )
+				if( o0 + 32 * b < ng ) v[b] = load_relaxed( q + dir * ( o0 + 32 * b ) );
+#pragma unroll
+			for( int b = 0; b < B; b++ )
+				if( o0 + 32 * b < ng )
+				{
+					list[dir * ( o0 + 32 * b )] = (int)(unsigned)v[b];
+					here = here && (unsigned)( v[b] >> 32 ) == tag;
+				}
+			if( !here ) // some stores are still on their way
+				for( int o = o0; o < min( ng, o0 + 32 * B ); o += 32 ) list[dir * o] = dense_id( tag, q + dir * o, load_relaxed( q + dir * o ) );
+		}
+	}
+}
+
+// seven rows into three planes (four full adders), added to the sums
+__device__ __forceinline__ void add_rows( unsigned ( &acc )[DN_SUM], unsigned x0, unsigned x1, unsigned x2, unsigned x3, unsigned x4, unsigned x5, unsigned x6 )
+{
+	unsigned const c1 = maj3( x0, x1, x2 ), s1 = x0 ^ x1 ^ x2;
+	unsigned const c2 = maj3( x3, x4, x5 ), s2 = x3 ^ x4 ^ x5;
+	unsigned const c3 = maj3( s1, s2, x6 ), ones = s1 ^ s2 ^ x6;
+	unsigned const fours = maj3( c1, c2, c3 ), twos = c1 ^ c2 ^ c3;
+	unsigned c = acc[0] & ones;
+	acc[0] ^= ones;
+	full_add( acc[1], twos, c );
+	full_add( acc[2], fours, c );
+#pragma unroll
+	for( int i = 3; i < DN_SUM; i++ )
+	{
+		unsigned const t = acc[i] & c;
+		acc[i] ^= c;
+		c = t;
+	}
+}
+
+// Count item: of round r's step s the arrivals of part `part`, in chunk u0 / DN_CHUNK of the
+// tile's units. A lane sums every eighth row's unit, seven rows at a time and the next seven
+// on their way; then the eight lanes of a unit add up, and each of the four that hold a
+// word's sums turns a quarter of its bit planes into bytes.
+// Long: steps whose ids are not in the list, or with more rows than a lane's planes count; a
+// form of its own, so that the other one's loop keeps its registers.
+constexpr int DN_PASS = 8 * ( ( 1 << DN_SUM ) - 1 ) / DN_ROWS * DN_ROWS; // rows whose sums fit a lane's planes
+template <int C, bool Long>
+__device__ __noinline__ void dense_count( int r, int s, int part, int u0 )
+{
+	dense_ctx & x = dense_get();
+	int const lane = threadIdx.x & 31, cap = x.cap;
+	int const c = part == 2 ? 1 : 0, nc = x.n[r & 3][s][c];
+	int const a0 = part == 1 ? ( nc + 1 ) >> 1 : 0, a1 = part == 0 ? ( nc + 1 ) >> 1 : nc;
+	int const dir = c ? -1 : 1, stride = (int)x.place.y, u = u0 + ( lane & 3 ), sub = lane >> 2;
+	int const * const list = dense_at<int>( x.ids ) + ( ( r & 1 ) * x.m + s ) * cap + ( c ? cap - 1 : 0 );
+	bool const active = u < x.units, upper = lane & 16;
+	uint2 const * const col = x.p.bits + x.place.x + ( active ? u : 0 );
+	constexpr int A = Long ? DN_OUT : DN_SUM + 3; // planes of the item's sums
+	unsigned a[A];
+#pragma unroll
+	for( int i = 0; i < A; i++ ) a[i] = 0u;
+	for( int p0 = a0; p0 < a1; p0 += DN_PASS )
+	{
+		int const end = Long ? min( a1, p0 + DN_PASS ) : a1;
+		unsigned ax[DN_SUM], ay[DN_SUM];
+#pragma unroll
+		for( int i = 0; i < DN_SUM; i++ ) ax[i] = ay[i] = 0u;
+		auto add7 = [&]( uint2 const ( &y )[7] ) {
+			add_rows( ax, y[0].x, y[1].x, y[2].x, y[3].x, y[4].x, y[5].x, y[6].x );
+			add_rows( ay, y[0].y, y[1].y, y[2].y, y[3].y, y[4].y, y[5].y, y[6].y );
+		};
+		if constexpr( !Long )
+		{
+			auto load = [&]( int e ) { return active && e < end ? load_row( col + (long long)list[dir * e] * stride ) : make_uint2( 0u, 0u ); };
+			uint2 y[7], z[7];
+#pragma unroll
+			for( int j = 0; j < 7; j++ ) y[j] = load( p0 + sub + 8 * j );
+			for( int e = p0; e < end; e += 2 * DN_ROWS )
+			{
+#pragma unroll
+				for( int j = 0; j < 7; j++ ) z[j] = load( e + DN_ROWS + sub + 8 * j );
+				add7( y );
+				if( e + DN_ROWS >= end ) break;
+#pragma unroll
+				for( int j = 0; j < 7; j++ ) y[j] = load( e + 2 * DN_ROWS + sub + 8 * j );
+				add7( z );
+			}
+		}
+		else
+		{
+			int const k = r * x.m + s - x.p.delay;
+			unsigned const tag = (unsigned)( x.t0 + k + 1 );
+			bool const listed = x.n[r & 3][s][0] + x.n[r & 3][s][1] <= cap;
+			int * const own = dense_at<int>( x.own ) + ( threadIdx.x >> 5 ) * DN_ROWS;
+#pragma unroll 1
+			for( int e = p0; e < end; e += DN_ROWS )
+			{
+				__syncwarp();
+#pragma unroll 1
+				for( int o = lane; o < min( DN_ROWS, end - e ); o += 32 )
+				{
+					unsigned long long const * q = dense_entry( k, c, e + o );
+					own[o] = listed ? list[dir * ( e + o )] : dense_id( tag, q, load_relaxed( q ) );
+				}
+				__syncwarp();
+				uint2 y[7];
+#pragma unroll
+				for( int j = 0; j < 7; j++ )
+					y[j] = active && e + sub + 8 * j < end ? load_row( col + (long long)own[sub + 8 * j] * stride ) : make_uint2( 0u, 0u );
+				add7( y );
+			}
+		}
+		// the two halves of the warp trade words, one of the two each, then add up the rest
+		unsigned b[DN_SUM + 3], carry = 0u;
+#pragma unroll
+		for( int i = 0; i < DN_SUM; i++ )
+		{
+			b[i] = upper ? ay[i] : ax[i];
+			full_add( b[i], __shfl_xor_sync( 0xffffffffu, upper ? ax[i] : ay[i], 16 ), carry );
+		}
+		b[DN_SUM] = carry;
+		carry = 0u;
+#pragma unroll
+		for( int i = 0; i <= DN_SUM; i++ ) full_add( b[i], __shfl_xor_sync( 0xffffffffu, b[i], 8 ), carry );
+		b[DN_SUM + 1] = carry;
+		carry = 0u;
+#pragma unroll
+		for( int i = 0; i <= DN_SUM + 1; i++ ) full_add( b[i], __shfl_xor_sync( 0xffffffffu, b[i], 4 ), carry );
+		b[DN_SUM + 2] = carry;
+		if constexpr( !Long )
+		{
+#pragma unroll
+			for( int i = 0; i < A; i++ ) a[i] = b[i];
+			break;
+		}
+		else
+		{
+			carry = 0u;
+#pragma unroll
+			for( int i = 0; i < A; i++ ) full_add( a[i], i < DN_SUM + 3 ? b[i] : 0u, carry );
+		}
+	}
+	// bytes of columns t, t + 8, t + 16, t + 24 of the word, t and t + 1
+	int const w = 2 * u + ( upper ? 1 : 0 ), t = ( lane >> 2 & 3 ) * 2, cols = x.cols;
+	unsigned char * const out = dense_at<unsigned char>( x.counts ) + ( ( ( r & 1 ) * x.m + s ) * dense_parts( C ) + part ) * 2 * cols + w * 32 + t * 4;
+	uint2 v = make_uint2( 0u, 0u );
+#pragma unroll
+	for( int i = 0; i < 8; i++ )
+	{
+		v.x |= ( ( a[i] >> t ) & 0x01010101u ) << i;
+		v.y |= ( ( a[i] >> ( t + 1 ) ) & 0x01010101u ) << i;
+	}
+	*reinterpret_cast<uint2 *>( out ) = v;
+	// the high bytes, which the update looks at once any part's are not zero
+	unsigned over = 0u;
+#pragma unroll
+	for( int i = 8; i < A; i++ ) over |= a[i];
+	v = make_uint2( 0u, 0u );
+	if( __any_sync( 0xffffffffu, over != 0u ) )
+	{
+		if( lane == 0 ) x.high[r & 3][s] = 1;
+#pragma unroll
+		for( int i = 8; i < A; i++ )
+		{
+			v.x |= ( ( a[i] >> t ) & 0x01010101u ) << ( i - 8 );
+			v.y |= ( ( a[i] >> ( t + 1 ) ) & 0x01010101u ) << ( i - 8 );
+		}
+	}
+	*reinterpret_cast<uint2 *>( out + cols ) = v;
+}
+
+// The window of CTA x.cta of a net: x.p, cta, L and dt are set, and visible to the CTA.
+template <typename Model>
+__device__ __forceinline__ void window_dense_body()
+{
+	dense_ctx & x = dense_get();
+	using N = typename Model::neuron;
+	constexpr int C = N::input_classes;
+	static_assert( C >= 1 && C <= DN_CLASSES, "window_dense keeps at most two input classes" );
+	int const tid = threadIdx.x, lane = tid & 31;
+	int const L = x.L;
+	bool const serial = x.p.delay < 3 || L <= 2;
+	int const m = serial ? min( L, dense_round( x.p.delay ) ) : dense_round( x.p.delay );
+	int const rounds = ( L + m - 1 ) / m;
+	int const tile_in = __ldg( x.p.cta_tiles + 2 * x.cta ), tile_free = __ldg( x.p.cta_tiles + 2 * x.cta + 1 );
+	int const d0_in = tile_in < 0 ? 0 : __ldg( x.p.tile_first + tile_in ), d0_free = tile_free < 0 ? 0 : __ldg( x.p.tile_first + tile_free );
+	int const span_in = tile_in < 0 ? 0 : __ldg( x.p.tile_first + tile_in + 1 ) - d0_in;
+	int const span_free = tile_free < 0 ? 0 : __ldg( x.p.tile_first + tile_free + 1 ) - d0_free;
+	dense_geom const geo = dense_layout( C, (int)N::size, span_in, span_free, m, x.p.delay );
+	int const list_ring = dense_ring( x.p.delay );
+	if( tid == 0 )
+	{
+		x.m = m;
+		x.tile[0] = tile_in;
+		x.tile[1] = tile_free;
+		x.d0[0] = d0_in;
+		x.d0[1] = d0_free;
+		x.span[0] = span_in;
+		x.span[1] = span_free;
+		for( int h = 0; h < 2; h++ )
+		{
+			x.words[h] = geo.words[h];
+			x.state[h] = (int)geo.state[h];
+			x.bits[h] = (int)geo.bits[h];
+		}
+		x.units = ( span_in + 63 ) >> 6;
+		x.chunks = ( x.units + DN_CHUNK - 1 ) / DN_CHUNK;
+		x.cols = x.chunks * DN_CHUNK * 64;
+		x.cap = DN_LIST / m;
+		x.words_before = (int)geo.words_before;
+		x.counts = (int)geo.counts;
+		x.ids = (int)geo.ids;
+		x.own = (int)geo.own;
+		if( tile_in >= 0 ) x.place = x.p.tile_place[tile_in];
+		clock_state const cs = *x.p.clock;
+		x.t0 = cs.step;
+		x.list_ring = list_ring;
+		x.slot0 = (int)( cs.step % x.p.ring );
+		x.list0 = (int)( cs.step % list_ring );
+		x.c = cs.c;
+		x.sum = cs.sum;
+		x.advance_clock( 0 );
+		for( int t = 0; t < 4; t++ ) x.queue[t] = 0u;
+	}
+	smem_state<N>::from_global( x.p.attr, d0_in, span_in, dense_at<unsigned char>( (int)geo.state[0] ) );
+	smem_state<N>::from_global( x.p.attr, d0_free, span_free, dense_at<unsigned char>( (int)geo.state[1] ) );
+	for( int y = tid; y < list_ring; y += DN_THREADS ) dense_at<unsigned long long>( (int)geo.words_before )[y] = x.p.step_before[y];
+	__syncthreads();
+
+	// Ticks. Overlapped: tick t publishes round t - 1, counts t + 1, scouts t + 2 and updates t.
+	// Serial, three ticks a round: publish the last and scout, count, update.
+	int const chunks = ( ( ( span_in + 63 ) >> 6 ) + DN_CHUNK - 1 ) / DN_CHUNK;
+	int const words_in = geo.words[0], words_free = geo.words[1];
+	int const end = serial ? 3 * rounds + 1 : rounds + 1;
+	for( int tick = serial ? 0 : -2; tick < end; tick++ )
+	{
+		int rp, rc, rs, ru;
+		if( serial )
+		{
+			int const r = tick / 3, stage = tick - 3 * r;
+			rp = stage == 0 ? r - 1 : -1;
+			rs = stage == 0 ? r : -1;
+			rc = stage == 1 ? r : -1;
+			ru = stage == 2 ? r : -1;
+		}
+		else
+		{
+			rp = tick - 1;
+			rc = tick + 1;
+			rs = tick + 2;
+			ru = tick;
+		}
+		auto in_run = [&]( int r ) { return r >= 0 && r < rounds; };
+		int const sc = in_run( rc ) ? x.steps( rc ) * chunks : 0; // count items of one part
+		int const np = in_run( rp ) ? x.steps( rp ) : 0, ns = in_run( rs ) ? x.steps( rs ) : 0;
+		int const nu = in_run( ru ) ? words_in : 0, nf = in_run( ru ) ? words_free : 0;
+		int const e0 = np, e1 = e0 + 2 * sc, e2 = e1 + ns, e3 = e2 + nu, e4 = e3 + nf, e5 = e4 + ( C > 1 ? sc : 0 );
+		for( ;; )
+		{
+			unsigned got = 0;
+			if( lane == 0 ) got = atomicAdd( x.queue + ( tick & 3 ), 1u );
+			int const item = (int)__shfl_sync( 0xffffffffu, got, 0 );
+			if( item >= e5 ) break;
+			if( item < e0 )
+				dense_publish<Model>( rp, item );
+			else if( item < e1 || item >= e4 )
+			{
+				// class 0 in halves first, class 1 last
+				int const part = item >= e4 ? 2 : ( item - e0 ) & 1, y = item >= e4 ? item - e4 : ( item - e0 ) >> 1;
+				int const s = y / chunks;
+				int const u0 = ( y - s * chunks ) * DN_CHUNK, a0 = x.n[rc & 3][s][0], a1 = x.n[rc & 3][s][1];
+				if( a0 + a1 > x.cap || ( part == 2 ? a1 : ( a0 + 1 ) >> 1 ) > DN_PASS )
+					dense_count<C, true>( rc, s, part, u0 );
+				else
+					dense_count<C, false>( rc, s, part, u0 );
+			}
+			else if( item < e2 )
+				dense_scout<C>( rs, item - e1 );
+			else if( item < e3 )
+				dense_update<Model>( ru, item - e2 );
+			else
+				dense_update_free<Model>( ru, item - e3 );
+			__syncwarp();
+		}
+		if( tid == 0 ) x.queue[( tick + 2 ) & 3] = 0u;
+		__syncthreads();
+	}
+	__syncthreads();
+	smem_state<N>::to_global( x.p.attr, d0_in, span_in, dense_at<unsigned char>( (int)geo.state[0] ) );
+	smem_state<N>::to_global( x.p.attr, d0_free, span_free, dense_at<unsigned char>( (int)geo.state[1] ) );
+	// the net's last CTA (batched launches run several nets) advances the clock and keeps the
+	// words before the steps: every CTA has read both
+	__syncthreads();
+	if( tid == 0 )
+	{
+		for( int h = 0; h < 2; h++ )
+			if( x.span[h] ) x.p.done_step[x.tile[h]] = x.t0 + L - 1;
+		__threadfence();
+		x.last = atomicAdd( &x.p.clock->done, 1u ) == (unsigned)x.p.nctas - 1;
+	}
+	__syncthreads();
+	if( !x.last ) return;
+	for( int y = tid; y < list_ring; y += DN_THREADS ) x.p.step_before[y] = dense_at<unsigned long long>( x.words_before )[y];
+	if( tid == 0 )
+	{
+		x.p.clock->step = x.t0 + L;
+		x.p.clock->c = x.c;
+		x.p.clock->sum = x.sum;
+		x.p.clock->done = 0;
+	}
+}
+
+// one net: CTA j runs its tiles cta_tiles[j]
+template <typename Model>
+__global__ void __launch_bounds__( DN_THREADS, 1 ) window_dense( net_params p, int L, float dt )
+{
+	dense_ctx & x = dense_get();
+	if( threadIdx.x == 0 )
+	{
+		x.p = p;
+		x.cta = blockIdx.x;
+		x.L = L;
+		x.dt = dt;
+	}
+	__syncthreads();
+	window_dense_body<Model>();
+}
+
+// Many independent nets of one model in one launch: jobs as window_flat_batch's, CTAs for tiles
+template <typename Model>
+__global__ void __launch_bounds__( DN_THREADS, 1 ) window_dense_batch( net_params const * nets, int4 const * jobs )
+{
+	dense_ctx & x = dense_get();
+	int4 const j = jobs[blockIdx.x];
+	if( j.z <= 0 ) return;
+	if( threadIdx.x == 0 )
+	{
+		x.p = nets[j.x];
+		x.cta = j.y;
+		x.L = j.z;
+		x.dt = __int_as_float( j.w );
+	}
+	__syncthreads();
+	window_dense_body<Model>();
+}
+} // namespace spk

@@ -81,6 +81,18 @@ struct net_params
 	int const * tile_in;
 	int tin, slot_vecs;
 	int * summ;
+	// target bitmaps (window_dense): tile j's first unit (64 targets) of source 0, and its
+	// units from source to source
+	uint2 const * bits;
+	longlong2 const * tile_place;
+	int const * cta_tiles; // [nctas][2] a CTA's tile with inputs and its tile without (-1: none)
+	int nctas;
+	// every step's spikes over all tiles, by class (window_dense): [3 delay][n] (step + 1) << 32 | id,
+	// [3 delay] tiles, spikes of class 1 and of class 0 added so far, and that word's value
+	// before its step
+	unsigned long long * step_ids;
+	unsigned long long * step_word;
+	unsigned long long * step_before;
 };
 
 template <typename T>

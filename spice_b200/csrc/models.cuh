@@ -63,6 +63,9 @@ constexpr bool is_plastic_model = Model::synapse::has_stdp;
 // no plasticity, no synapse attributes (the counts replay knows only the source's class)
 template <typename Model>
 constexpr bool is_flat_model = Model::neuron::input_classes > 0 && !Model::synapse::has_stdp && Model::synapse::size == 0;
+// models window_dense runs too: its lists hold at most two input classes
+template <typename Model>
+constexpr bool is_dense_model = is_flat_model<Model> && Model::neuron::input_classes <= 2;
 // models that only the generic kernel (window_ordered) runs: the other non-plastic ones
 template <typename Model>
 constexpr bool needs_ordered = !Model::synapse::has_stdp && !is_flat_model<Model>;

@@ -6,6 +6,7 @@
 // window); spk_net_run replays a captured CUDA graph of many windows.
 #include "kernels.cuh"
 #include "flat.cuh"
+#include "dense.cuh"
 #include "models.cuh"
 #include "ordered.cuh"
 #include "plastic.cuh"
@@ -406,6 +407,7 @@ struct build_opts
 	bool direct = false;   // per-step kernels instead of the window kernels
 	bool kernel_auto = true; // the kernel is the automatic choice (no field value, no test override)
 	bool ordered = false;  // the generic window_ordered kernel for any non-plastic model
+	bool bitmaps = true;   // target bitmaps where a net is dense enough (no slice width asked for)
 	bool pack16 = false;   // 16-bit slice indices even where 10-bit ones fit
 	bool uniform = false;  // equal tiles instead of cost-balanced ones
 	bool windowed = false; // no persistent launch
@@ -439,6 +441,7 @@ build_opts resolve_opts( spk_net_options const * o )
 	r.direct = kernel == 1;
 	r.kernel_auto = d.kernel < 0 && !ke;
 	r.ordered = kernel == 2;
+	r.bitmaps = d.slice_bits < 0 && !getenv( "SPK_PACK" ) && d.pipelined < 0 && !getenv( "SPK_FLAT_SYNC" );
 	r.pack16 = d.slice_bits >= 0 ? d.slice_bits == 16 : env_is( "SPK_PACK", "16" );
 	r.uniform = pick( d.tiling, "SPK_TILES", "uniform", "balanced", false );
 	r.windowed = !pick( d.persistent, "SPK_PERSIST", "1", "0", true );
@@ -512,6 +515,12 @@ struct spk_net
 	int slot_vecs = 0, tin = 0;
 	int slot_smem = 0; // dynamic shared memory of a window_slots launch
 	dbuf slot_data, tile_in, summ;
+	// window_dense (dense.cuh): the rows as target bitmaps instead of slices
+	bool dense = false;
+	int row_units = 0;
+	int dense_smem = 0; // dynamic shared memory of a window_dense launch
+	int nctas = 0; // CTAs of a window_dense launch
+	dbuf row_bits, tile_place, cta_tiles, step_ids, step_word, step_before;
 	bool persistent = false; // run() as one cooperative window_flat launch (delay >= 6)
 	// failure-detection tests (SPK_TEST_WAIT_LIMIT, SPK_TEST_WITHHOLD_TILE at creation): a
 	// shorter bounded wait, and a tile that never publishes its steps so that the waits of
@@ -563,6 +572,13 @@ struct spk_net
 		p.tin = tin;
 		p.slot_vecs = slot_vecs;
 		p.summ = summ.as<int>();
+		p.bits = row_bits.as<uint2 const>();
+		p.tile_place = tile_place.as<longlong2 const>();
+		p.cta_tiles = cta_tiles.as<int const>();
+		p.nctas = nctas;
+		p.step_ids = step_ids.as<unsigned long long>();
+		p.step_word = step_word.as<unsigned long long>();
+		p.step_before = step_before.as<unsigned long long>();
 		return p;
 	}
 
@@ -571,18 +587,21 @@ struct spk_net
 		size_t b = edges.bytes + pivots.bytes + tile_first.bytes + ring_ids.bytes + ring_cnt.bytes + clock.bytes + dt_ring.bytes + err.bytes +
 		           conns_dev.bytes + gather_ids.bytes + gather_cnt.bytes + cursor.bytes + gather_done.bytes + rec_ids.bytes +
 		           rec_cnt.bytes + plast.bytes() + slices.bytes + slice_rec.bytes + tile_inputs.bytes + done_step.bytes +
-		           slot_data.bytes + tile_in.bytes + summ.bytes;
+		           slot_data.bytes + tile_in.bytes + summ.bytes + row_bits.bytes + tile_place.bytes + cta_tiles.bytes +
+		           step_ids.bytes + step_word.bytes + step_before.bytes;
 		for( auto const & a : attr ) b += a.bytes;
 		for( auto const & a : syn ) b += a.bytes;
 		return b;
 	}
 
+	// CTAs of a window launch: one per tile, or per pair of tiles
+	int ctas() const { return dense ? nctas : tc.ntiles; }
 	int classes() const { return classes_of( model ); }
 	int neuron_attrs() const { return neuron_attrs_of( model ); }
 
 	int window_smem() const
 	{
-		if( flat ) return slot_vecs ? slot_smem : flat_smem;
+		if( flat ) return slot_vecs ? slot_smem : dense ? dense_smem : flat_smem;
 		int const classes = this->classes();
 		size_t const head = ( (size_t)classes * tc.tile + tc.ntiles + 1 ) * 4;
 		size_t b = ( ( head + 15 ) & ~(size_t)15 ) + (size_t)spk::SPIKE_BATCH * 16;
@@ -649,15 +668,30 @@ struct spk_net
 				slot_smem = optin - (int)std::max( fs.sharedSizeBytes, fsb.sharedSizeBytes );
 				set_smem_limit( (void const *)spk::window_slots<Model>, device, slot_smem );
 				set_smem_limit( (void const *)spk::window_slots_batch<Model>, device, slot_smem );
+				if constexpr( spk::is_dense_model<Model> )
+					if( dense )
+					{
+						cudaFuncAttributes fd{}, fdb{};
+						CK( cudaFuncGetAttributes( &fd, spk::window_dense<Model> ) );
+						CK( cudaFuncGetAttributes( &fdb, spk::window_dense_batch<Model> ) );
+						dense_smem = optin - (int)std::max( fd.sharedSizeBytes, fdb.sharedSizeBytes );
+						set_smem_limit( (void const *)spk::window_dense<Model>, device, dense_smem );
+						set_smem_limit( (void const *)spk::window_dense_batch<Model>, device, dense_smem );
+					}
 				// one launch for a whole run: every tile's CTA resident at once (cooperative
 				// launch), and the step pipeline never waits on a step not yet simulated
 				int coop = 0, per_sm = 0;
 				CK( cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, device ) );
 				if( slot_vecs )
 					CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, spk::window_slots<Model>, tc.threads, slot_smem ) );
+				else if( dense )
+				{
+					if constexpr( spk::is_dense_model<Model> )
+						CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, spk::window_dense<Model>, spk::DN_THREADS, dense_smem ) );
+				}
 				else
 					CK( cudaOccupancyMaxActiveBlocksPerMultiprocessor( &per_sm, spk::window_flat<Model>, tc.threads, flat_smem ) );
-				persistent = coop && (long long)per_sm * sms >= tc.ntiles && !opts.windowed;
+				persistent = coop && (long long)per_sm * sms >= ctas() && !opts.windowed;
 				return;
 			}
 		// the limit is per kernel, shared by every net: set it to all a CTA can have, so a
@@ -702,6 +736,11 @@ struct spk_net
 			{
 				if( slot_vecs )
 					spk::window_slots<Model><<<tc.ntiles, tc.threads, smem, stream>>>( p, L, dt, smem );
+				else if( dense )
+				{
+					if constexpr( spk::is_dense_model<Model> )
+						spk::window_dense<Model><<<nctas, spk::DN_THREADS, smem, stream>>>( p, L, dt );
+				}
 				else
 					spk::window_flat<Model><<<tc.ntiles, tc.threads, smem, stream>>>( p, L, dt, smem );
 			}
@@ -833,11 +872,13 @@ struct spk_net
 			// shorter delays run every step on the synchronous path (each step waits for the
 			// steps it reads). window_slots looks five steps ahead (its nets have delay >= 7).
 			if( !slot_vecs && delay < 6 ) p.flat_sync = 1;
-			int smem = slot_vecs ? slot_smem : flat_smem;
+			int smem = window_smem();
 			float d = dt;
 			void * args[] = { &p, &L, &d, &smem };
 			void const * kernel = slot_vecs ? (void const *)spk::window_slots<Model> : (void const *)spk::window_flat<Model>;
-			CK( cudaLaunchCooperativeKernel( kernel, dim3( tc.ntiles ), dim3( tc.threads ), args, (size_t)smem, stream ) );
+			if constexpr( spk::is_dense_model<Model> )
+				if( dense ) kernel = (void const *)spk::window_dense<Model>; // takes the first three
+			CK( cudaLaunchCooperativeKernel( kernel, dim3( ctas() ), dim3( dense ? spk::DN_THREADS : tc.threads ), args, (size_t)smem, stream ) );
 		}
 	}
 	void launch_persistent( int L )
@@ -1053,21 +1094,135 @@ void set_tiles( spk_net & net, std::vector<int> const & first )
 	CK( cudaStreamSynchronize( net.stream ) );
 }
 
+// the tiles that hold a neuron with inputs
+std::vector<char> input_tiles( std::vector<cost_segment> const & segs, std::vector<int> const & first )
+{
+	std::vector<char> in( first.size() - 1, 0 );
+	size_t si = 0;
+	for( size_t i = 0; i + 1 < first.size(); i++ )
+	{
+		while( si + 1 < segs.size() && segs[si + 1].start <= first[i] ) si++;
+		for( size_t k = si; k < segs.size() && segs[k].start < first[i + 1]; k++ ) in[i] |= segs[k].cost > UPDATE_COST;
+	}
+	return in;
+}
+
+// window_dense's CTAs: the i-th tile with inputs and the i-th tile without
+std::vector<std::pair<int, int>> pair_tiles( std::vector<char> const & has_inputs )
+{
+	std::vector<int> in, free;
+	for( size_t j = 0; j < has_inputs.size(); j++ ) ( has_inputs[j] ? in : free ).push_back( (int)j );
+	std::vector<std::pair<int, int>> c( std::max( in.size(), free.size() ) );
+	for( size_t i = 0; i < c.size(); i++ ) c[i] = { i < in.size() ? in[i] : -1, i < free.size() ? free[i] : -1 };
+	return c;
+}
+
+// Whether window_dense takes a net of `syn` synapses on this tiling: the tiles with inputs
+// within its limits and its shared memory, and the bitmaps at most DENSE_MAX_RATIO times the
+// bytes of the index lists, or DENSE_WIDE_RATIO times in tiles of more than DENSE_WIDE
+// neurons. The work of a bitmap row grows with its tile, that of a list with its synapses:
+// at p = 0.02 (ratio 2.2 to 2.5) VA of 70,710 and 100,000 neurons (tiles of 478 and 676) takes
+// 2.18 and 3.33 us per step against 4.01 and 4.00 with lists, of 223,607 (1,511) 11.8
+// against 7.3-11.8; at p = 0.05 100,000 neurons 2.4-2.7 against 4.3-5.5.
+constexpr double DENSE_MAX_RATIO = 3.0, DENSE_WIDE_RATIO = 1.2;
+constexpr int DENSE_WIDE = 1024;
+bool dense_fits( int model, int device, long long n, int delay, double syn, double max_in, std::vector<int> const & first, std::vector<char> const & has_inputs, int pack )
+{
+	int const classes = classes_of( model ), attrs = neuron_attrs_of( model );
+	if( classes < 1 || classes > spk::DN_CLASSES || syn <= 0 || n >= spk::DN_MAX_N || max_in > spk::DN_MAX_IN ) return false;
+	int optin = 0;
+	CK( cudaDeviceGetAttribute( &optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device ) );
+	size_t const smem = (size_t)optin - 4096; // the kernels' static shared memory
+	int const m = spk::dense_round( delay );
+	double units = 0, tiles = 0;
+	int widest = 0;
+	for( auto const & c : pair_tiles( has_inputs ) )
+	{
+		int const in = c.first < 0 ? 0 : first[c.first + 1] - first[c.first], free = c.second < 0 ? 0 : first[c.second + 1] - first[c.second];
+		if( in > spk::DN_MAX_TILE || spk::dense_layout( classes, attrs, in, free, m, delay ).end > smem ) return false;
+		if( in ) units += spk::dense_units( in );
+		tiles += in > 0;
+		widest = std::max( widest, in );
+	}
+	if( units * 8 > 96 * 1024 ) return false; // a row is built in shared memory
+	double const slices = syn / n * 16 / pack + 16 * tiles;
+	return units * 8 <= ( widest > DENSE_WIDE ? DENSE_WIDE_RATIO : DENSE_MAX_RATIO ) * slices;
+}
+
+// window_dense's tiling: at most about `target` tiles with inputs of about equal cost (a
+// neuron's update and replay, and its share of the counting, grow with its in-degree), and
+// as many without, both of at least DENSE_MIN_TILE neurons: a smaller tile's row parts fill
+// no sector.
+constexpr int DENSE_MIN_TILE = 256;
+std::vector<int> dense_tiles( std::vector<cost_segment> const & segs, long long n, int target, int tmax_in, int tmax_free )
+{
+	auto seg_end = [&]( size_t i ) { return i + 1 < segs.size() ? segs[i + 1].start : n; };
+	auto is_free = [&]( size_t i ) { return segs[i].cost <= UPDATE_COST; };
+	double total[2] = { 0, 0 }, count[2] = { 0, 0 };
+	for( size_t i = 0; i < segs.size(); i++ )
+	{
+		total[is_free( i )] += ( seg_end( i ) - segs[i].start ) * segs[i].cost;
+		count[is_free( i )] += (double)( seg_end( i ) - segs[i].start );
+	}
+	double share[2];
+	for( int k = 0; k < 2; k++ ) share[k] = std::max( total[k] / target, total[k] / std::max( 1.0, count[k] ) * DENSE_MIN_TILE );
+	std::vector<int> first;
+	for( int it = 0; it < 400; it++ )
+	{
+		int tiles[2] = { 0, 0 };
+		first.assign( 1, 0 );
+		long long start = 0;
+		double acc = 0;
+		auto close = [&]( long long at, int kind ) {
+			if( at == start ) return;
+			tiles[kind]++;
+			first.push_back( (int)at );
+			start = at;
+			acc = 0;
+		};
+		for( size_t i = 0; i < segs.size(); i++ )
+		{
+			int const kind = is_free( i ), tmax = kind ? tmax_free : tmax_in;
+			if( i > 0 && is_free( i - 1 ) != is_free( i ) ) close( segs[i].start, is_free( i - 1 ) );
+			for( long long pos = segs[i].start; pos < seg_end( i ); )
+			{
+				long long const fit = std::max( 1LL, (long long)std::ceil( ( share[kind] - acc ) / segs[i].cost - 1e-9 ) );
+				long long const take = std::min( { seg_end( i ) - pos, fit, tmax - ( pos - start ) } );
+				pos += take;
+				acc += take * segs[i].cost;
+				if( acc >= share[kind] * ( 1 - 1e-12 ) || pos - start >= tmax ) close( pos, kind );
+			}
+		}
+		close( n, is_free( segs.size() - 1 ) );
+		bool const ok[2] = { tiles[0] <= target, tiles[1] <= target };
+		if( ok[0] && ok[1] ) break;
+		for( int k = 0; k < 2; k++ )
+			if( !ok[k] ) share[k] *= 1.01;
+	}
+	return first;
+}
+
 // window_flat's tiling of n neurons into at most about `target` work-balanced tiles (target
 // = the SM count for a net alone; fewer for a net that shares the GPU in a batch): the
 // tiles' first neurons and the shared-memory span of the largest tile with inputs; false
-// if the net does not fit window_flat.
+// if the net does not fit window_flat. `dense`: the tiling is window_dense's (for a net alone:
+// in the windows of shared launches every launch fills and drains its rounds, and the lists
+// are the faster: 24 nets of three models 20.2 ms for 600 steps, with bitmaps 22.2).
 bool plan_flat( int model,
                 int device,
                 long long n,
                 long long width,
+                int delay,
                 std::vector<cost_segment> const & segs,
                 int target,
+                bool alone,
                 build_opts const & o,
                 std::vector<int> & first,
                 int & span,
-                int & pack )
+                int & pack,
+                bool & dense )
 {
+	dense = false;
 	int optin = 0;
 	CK( cudaDeviceGetAttribute( &optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device ) );
 	int const classes = classes_of( model ), attrs = neuron_attrs_of( model );
@@ -1120,16 +1275,38 @@ bool plan_flat( int model,
 			}
 		}
 	}
+	// target bitmaps instead of slices
+	if( alone && o.bitmaps && !o.slots && classes <= spk::DN_CLASSES )
+	{
+		// a pair's tiles share the CTA: half of it for a tile without inputs
+		int const dfree = (int)( ( optin / 2 ) / ( 4.0 * attrs + 2 * spk::DN_MB / 8.0 ) ) / 64 * 64;
+		auto const f = uniform ? uniform_tiles( n, 1024 )
+		                       : dense_tiles( segs, n, std::max( 1, target ), std::min( tmax, spk::DN_MAX_TILE ), std::min( tmax_free, dfree ) );
+		std::vector<char> const in = input_tiles( segs, f );
+		double max_in = 0; // expected
+		for( auto const & c : segs ) max_in = std::max( max_in, c.cost - UPDATE_COST );
+		if( f.size() < (size_t)spk::FLAT_PC && dense_fits( model, device, n, delay, segment_synapses( segs, n ), max_in + 8 * std::sqrt( max_in ), f, in, pack ) )
+		{
+			dense = true;
+			first = f;
+			span = 0;
+			for( size_t i = 0; i + 1 < f.size(); i++ )
+				if( in[i] ) span = std::max( span, f[i + 1] - f[i] );
+			pack = (long long)classes * ( ( span + 31 ) / 32 * 32 ) < (long long)spk::SLICE_PAD10 ? 12 : 8;
+		}
+	}
 	return true;
 }
 
 // plan_flat applied to a net: sets net.flat and the tiles
-bool flat_tiling( spk_net & net, std::vector<cost_segment> const & segs, int target )
+bool flat_tiling( spk_net & net, std::vector<cost_segment> const & segs, int target, bool alone )
 {
 	std::vector<int> first;
 	int span = 0, pack = 8;
-	if( !plan_flat( net.model, net.device, net.n, net.width, segs, target, net.opts, first, span, pack ) ) return false;
+	bool dense = false;
+	if( !plan_flat( net.model, net.device, net.n, net.width, net.delay, segs, target, alone, net.opts, first, span, pack, dense ) ) return false;
 	net.flat = true;
+	net.dense = dense;
 	net.pack = pack;
 	net.flat_tmax = ( span + 31 ) / 32 * 32;
 	net.tc = { spk::FLAT_THREADS, 1, net.flat_tmax, (int)first.size() - 1 };
@@ -1168,7 +1345,7 @@ void allocate( spk_net & net, long long n, long long width, std::vector<cost_seg
 	net.flat = false;
 	int const target = net.opts.tile_target;
 	bool const per_step = net.opts.kernel_auto && net.delay == 1 && segment_synapses( segs, n ) <= PER_STEP_MAX_SYNAPSES;
-	if( !md.plastic && !net.ordered && !net.opts.direct && !per_step ) flat_tiling( net, segs, target > 0 ? target : dev_sms );
+	if( !md.plastic && !net.ordered && !net.opts.direct && !per_step ) flat_tiling( net, segs, target > 0 ? target : dev_sms, target == 0 );
 	if( !net.flat ) set_tiles( net, uniform_tiles( n, net.tc.tile ) );
 	net.ring_slots = 2 * net.delay;
 	allocate_buffers( net );
@@ -1297,9 +1474,91 @@ bool plan_slots( spk_net & net )
 	return true;
 }
 
+// Tiles whose parts of a row lie together. One tile each: rows of 64 bytes, at 1e9 synapses
+// 4.13 us per step; four 3.76, sixteen 3.77, all of them (a row in one stretch, every tile
+// reading over the whole 1.3 GB) 3.91.
+constexpr size_t DENSE_GROUP = 4;
+
+// the target bitmaps of window_dense, from the ELL rows
+void build_bitmaps( spk_net & net )
+{
+	int const nt = net.tc.ntiles;
+	long long const n = net.n;
+	net.tile_inputs.alloc( (size_t)nt * 4, net.mem() );
+	net.tile_place.alloc( (size_t)nt * sizeof( longlong2 ), net.mem() );
+	net.done_step.alloc( (size_t)nt * sizeof( long long ), net.mem() );
+	CK( cudaMemsetAsync( net.tile_inputs.p, 0, net.tile_inputs.bytes, net.stream ) );
+	CK( cudaMemsetAsync( net.done_step.p, 0xFF, net.done_step.bytes, net.stream ) ); // -1: nothing published
+	int const rows = (int)std::min<long long>( 8 * net.sms, ( n * 32 + 255 ) / 256 );
+	spk::dense_tile_inputs<<<rows, 256, 0, net.stream>>>( (int)n, nt, net.pivots.as<unsigned>(), net.tile_inputs.as<int>() );
+	CK( cudaGetLastError() );
+	std::vector<int> in( nt ), unit( nt, 0 );
+	CK( cudaMemcpyAsync( in.data(), net.tile_inputs.p, (size_t)nt * 4, cudaMemcpyDeviceToHost, net.stream ) );
+	CK( cudaStreamSynchronize( net.stream ) );
+	net.row_units = 0;
+	for( int j = 0; j < nt; j++ )
+	{
+		unit[j] = net.row_units;
+		if( in[j] ) net.row_units += spk::dense_units( net.tile_first_host[j + 1] - net.tile_first_host[j] );
+	}
+	if( net.row_units == 0 ) net.row_units = 4; // a net that drew no synapse
+	std::vector<int> cta;
+	for( auto const & c : pair_tiles( std::vector<char>( in.begin(), in.end() ) ) )
+	{
+		cta.push_back( c.first );
+		cta.push_back( c.second );
+	}
+	net.nctas = (int)cta.size() / 2;
+	net.cta_tiles.alloc( cta.size() * 4, net.mem() );
+	CK( cudaMemcpyAsync( net.cta_tiles.p, cta.data(), cta.size() * 4, cudaMemcpyHostToDevice, net.stream ) );
+	net.row_bits.alloc( (size_t)n * net.row_units * 8, net.mem() );
+	int const ring = spk::dense_ring( net.delay );
+	net.step_ids.alloc( (size_t)ring * n * 8, net.mem() );
+	net.step_word.alloc( (size_t)ring * 8, net.mem() );
+	net.step_before.alloc( (size_t)ring * 8, net.mem() );
+	// ids start as a valid neuron id (see ring_ids)
+	CK( cudaMemsetAsync( net.step_ids.p, 0, net.step_ids.bytes, net.stream ) );
+	CK( cudaMemsetAsync( net.step_word.p, 0, net.step_word.bytes, net.stream ) );
+	CK( cudaMemsetAsync( net.step_before.p, 0, net.step_before.bytes, net.stream ) );
+	// the tiles with inputs in groups of DENSE_GROUP: a group's parts of a row lie together
+	std::vector<longlong2> place( nt, longlong2{ 0, 0 } ), chunk;
+	std::vector<int> with;
+	for( int j = 0; j < nt; j++ )
+		if( in[j] ) with.push_back( j );
+	for( size_t g = 0; g < with.size(); g += DENSE_GROUP )
+	{
+		size_t const e = std::min( with.size(), g + DENSE_GROUP );
+		int const last = with[e - 1];
+		long long const from = unit[with[g]], stride = unit[last] + spk::dense_units( net.tile_first_host[last + 1] - net.tile_first_host[last] ) - from;
+		for( size_t i = g; i < e; i++ ) place[with[i]] = longlong2{ n * from + ( unit[with[i]] - from ), stride };
+		for( long long c = 0; c < stride; c += 4 ) chunk.push_back( longlong2{ n * from + c, stride } );
+	}
+	if( chunk.empty() ) chunk.push_back( longlong2{ 0, 4 } );
+	sbuf pos( (size_t)n * 4, net.stream, net.device ), unit_dev( (size_t)nt * 4, net.stream, net.device ),
+	    chunk_dev( chunk.size() * sizeof( longlong2 ), net.stream, net.device );
+	CK( cudaMemcpyAsync( unit_dev.p, unit.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, net.stream ) );
+	CK( cudaMemcpyAsync( chunk_dev.p, chunk.data(), chunk.size() * sizeof( longlong2 ), cudaMemcpyHostToDevice, net.stream ) );
+	CK( cudaMemcpyAsync( net.tile_place.p, place.data(), (size_t)nt * sizeof( longlong2 ), cudaMemcpyHostToDevice, net.stream ) );
+	spk::dense_positions<<<(int)( ( n + 255 ) / 256 ), 256, 0, net.stream>>>( (int)n, nt, net.tile_first.as<int>(), unit_dev.as<int>(), pos.as<int>() );
+	CK( cudaGetLastError() );
+	int const smem = net.row_units * 8;
+	set_smem_limit( (void const *)spk::dense_fill, net.device, 96 * 1024 );
+	spk::dense_fill<<<(int)std::min<long long>( n, 16LL * net.sms ), 512, smem, net.stream>>>(
+	    (int)n, (int)net.width, net.row_units, net.edges.as<int>(), pos.as<int>(), chunk_dev.as<longlong2>(), net.row_bits.as<uint2>() );
+	CK( cudaGetLastError() );
+	CK( cudaStreamSynchronize( net.stream ) ); // the host tables are freed on return
+	net.configure(); // whether its CTAs are resident at once
+}
+
 // the tile-major slices of window_flat, from the ELL rows and their pivots
 void build_slices( spk_net & net )
 {
+	if( net.dense )
+	{
+		build_bitmaps( net );
+		return;
+	}
+	for( dbuf * b : { &net.row_bits, &net.tile_place, &net.cta_tiles, &net.step_ids, &net.step_word, &net.step_before } ) b->reset(); // of an earlier tiling
 	int const nt = net.tc.ntiles;
 	long long const n = net.n;
 	net.slice_rec.alloc( (size_t)n * nt * sizeof( uint2 ), net.mem() );
@@ -1365,7 +1624,7 @@ void retile( spk_net & net, int target )
 	std::vector<cost_segment> segs;
 	for( size_t i = 0; i < net.seg_start.size(); i++ ) segs.push_back( { (long long)net.seg_start[i], net.seg_cost[i] } );
 	CK( cudaStreamSynchronize( net.stream ) );
-	require( flat_tiling( net, segs, target ), "tiling failed" );
+	require( flat_tiling( net, segs, target, false ), "tiling failed" );
 	net.pivots.alloc( (size_t)net.n * ( net.tc.ntiles + 1 ) * 4, net.mem() );
 	net.ring_cnt.alloc( (size_t)net.ring_slots * net.tc.ntiles * 4, net.mem() );
 	CK( cudaMemsetAsync( net.ring_cnt.p, 0, net.ring_cnt.bytes, net.stream ) );
@@ -1429,9 +1688,10 @@ size_t estimate_bytes( int model, spice::util::layout const & l, int delay, int 
 	CK( cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, device ) );
 	spk::model_traits const md = describe( model );
 	int const attrs = md.neuron_attrs;
-	bool flat = false;
+	bool flat = false, dense = false;
 	long long T = 0;
 	int pack = 8;
+	double units = 0;
 	if( !md.plastic && ( md.ordered || o.ordered ) )
 		T = choose_tiles( n, sms, spk::ORD_MAX_TILE, 2 ).ntiles;
 	else if( !md.plastic )
@@ -1440,10 +1700,13 @@ size_t estimate_bytes( int model, spice::util::layout const & l, int delay, int 
 		int span = 0;
 		std::vector<cost_segment> const segs = layout_costs( l );
 		bool const per_step = o.kernel_auto && delay == 1 && segment_synapses( segs, n ) <= PER_STEP_MAX_SYNAPSES;
-		if( !o.direct && !per_step && plan_flat( model, device, n, w, segs, o.tile_target > 0 ? o.tile_target : sms, o, first, span, pack ) )
+		if( !o.direct && !per_step && plan_flat( model, device, n, w, delay, segs, o.tile_target > 0 ? o.tile_target : sms, o.tile_target == 0, o, first, span, pack, dense ) )
 		{
 			flat = true;
 			T = (long long)first.size() - 1;
+			std::vector<char> const in = input_tiles( segs, first );
+			for( size_t i = 0; i + 1 < first.size(); i++ )
+				if( in[i] ) units += spk::dense_units( first[i + 1] - first[i] );
 		}
 		else
 			T = choose_tiles( n, sms, 2048, 4 ).ntiles;
@@ -1465,7 +1728,16 @@ size_t estimate_bytes( int model, spice::util::layout const & l, int delay, int 
 	for( int i = 0; i < attrs; i++ ) b.push_back( (double)n * 4 );
 	if( !md.plastic )
 		for( int i = 0; i < md.synapse_attrs; i++ ) b.push_back( (double)n * w * 4 );
-	if( flat )
+	if( flat && dense )
+	{
+		b.push_back( (double)n * std::max( units, 4.0 ) * 8 );
+		b.push_back( (double)n * 4 ); // the targets' bit positions, while the bitmaps are built
+		b.push_back( (double)spk::dense_ring( delay ) * n * 8 );
+		for( int i = 0; i < 2; i++ ) b.push_back( (double)spk::dense_ring( delay ) * 8 );
+		b.push_back( (double)T * 4 );
+		for( int i = 0; i < 3; i++ ) b.push_back( (double)T * 16 );
+	}
+	else if( flat )
 	{
 		b.push_back( (double)n * T * 8 );
 		b.push_back( 16.0 * ( std::ceil( syn / pack ) + std::min( (double)n * T, syn ) ) );
@@ -1566,7 +1838,9 @@ std::vector<T> ckpt_read( ckpt_dir const & dir, uint32_t id, uint64_t count )
 	if( count ) std::memcpy( v.data(), ckpt_find( dir, id, count * sizeof( T ) ), count * sizeof( T ) );
 	return v;
 }
-void validate_checkpoint( ckpt_header const & h, std::vector<int> const & first, ckpt_dir const & dir )
+// syn, max_in, in_tile: the graph's synapses, its largest in-degree and the tiles that receive
+// any.
+void validate_checkpoint( ckpt_header const & h, std::vector<int> const & first, ckpt_dir const & dir, double & syn, double & max_in, std::vector<char> & in_tile )
 {
 	uint64_t const n = (uint64_t)h.n, width = (uint64_t)h.width;
 	int const T = h.ntiles;
@@ -1586,12 +1860,16 @@ void validate_checkpoint( ckpt_header const & h, std::vector<int> const & first,
 		}
 		validate_edges( e, n, width );
 		// tiles that receive synapses
-		std::vector<char> in_tile( T, 0 );
-		std::vector<char> target( n, 0 );
+		std::vector<int> target( n, 0 );
 		for( uint64_t k = 0; k < n * width; k++ )
-			if( e[k] != INT_MAX ) target[e[k]] = 1;
+			if( e[k] != INT_MAX )
+			{
+				target[e[k]]++;
+				syn++;
+			}
+		for( int t : target ) max_in = std::max<double>( max_in, t );
 		for( int j = 0; j < T; j++ )
-			for( int d = first[j]; d < first[j + 1] && !in_tile[j]; d++ ) in_tile[j] = target[d];
+			for( int d = first[j]; d < first[j + 1] && !in_tile[j]; d++ ) in_tile[j] = target[d] > 0;
 		if( h.flat == 1 )
 		{
 			unsigned const pad = h.pack == 12 ? spk::SLICE_PAD10 : spk::SLICE_PAD;
@@ -1751,8 +2029,8 @@ struct spk_batch
 	// by model id and kernel: window_flat, window_slots, window_plastic (one CTA per SM, up to
 	// 512 threads), then window_plastic in its two-CTAs-per-SM form for tiles of 257 to
 	// PL_THREADS, up to 128 and 129 to 256 neurons (a launch is as wide as its widest tile:
-	// narrow tiles in narrow launches, so several of their CTAs share an SM)
-	static constexpr int KINDS = 6;
+	// narrow tiles in narrow launches, so several of their CTAs share an SM); 6: window_dense
+	static constexpr int KINDS = 7;
 	group groups[KINDS * spk::MODEL_COUNT];
 
 	~spk_batch()
@@ -1776,7 +2054,7 @@ struct spk_batch
 			int const w = net.tc.threads;
 			return w <= 128 ? 4 : w <= 256 ? 5 : w <= spk::PL_THREADS ? 3 : 2;
 		}
-		return net.slot_vecs ? 1 : 0;
+		return net.slot_vecs ? 1 : net.dense ? 6 : 0;
 	}
 
 	template <typename Model>
@@ -1787,6 +2065,11 @@ struct spk_batch
 		{
 			if( kind == 1 )
 				spk::window_slots_batch<Model><<<njobs, spk::FLAT_THREADS, smem, g.stream>>>( params, jobs, smem );
+			else if( kind == 6 )
+			{
+				if constexpr( spk::is_dense_model<Model> )
+					spk::window_dense_batch<Model><<<njobs, spk::DN_THREADS, smem, g.stream>>>( params, jobs );
+			}
 			else
 				spk::window_flat_batch<Model><<<njobs, spk::FLAT_THREADS, smem, g.stream>>>( params, jobs, smem );
 			CK( cudaGetLastError() );
@@ -1814,7 +2097,7 @@ struct spk_batch
 		}
 		g.h_params.resize( gn.size() );
 		for( size_t i = 0; i < gn.size(); i++ ) g.h_params[i] = gn[i]->params();
-		bool const plastic = kind >= 2;
+		bool const plastic = kind >= 2 && kind <= 5;
 		g.h_pls.resize( plastic ? gn.size() : 0 );
 		for( size_t i = 0; i < g.h_pls.size(); i++ ) g.h_pls[i] = gn[i]->plast.params();
 		// all rounds' jobs (net, tile, steps, dt) at once; a round whose windows equal the
@@ -1838,7 +2121,7 @@ struct spk_batch
 					{
 						int dtbits;
 						std::memcpy( &dtbits, &gn[i]->dt, 4 );
-						for( int j = 0; j < gn[i]->tc.ntiles; j++ ) g.h_jobs.push_back( make_int4( (int)i, j, L[i], dtbits ) );
+						for( int j = 0; j < gn[i]->ctas(); j++ ) g.h_jobs.push_back( make_int4( (int)i, j, L[i], dtbits ) );
 					}
 				launches.push_back( { first, (int)g.h_jobs.size() - first } );
 				prevL = L;
@@ -1886,7 +2169,7 @@ struct spk_batch
 		}
 		// launch shape: window_flat's fixed one, or the widest plastic tile and the largest
 		// shared-memory carve-up at that width
-		int threads = spk::FLAT_THREADS, smem = kind == 1 ? gn[0]->slot_smem : gn[0]->flat_smem;
+		int threads = spk::FLAT_THREADS, smem = gn[0]->window_smem();
 		if( plastic )
 		{
 			threads = 32;
@@ -2362,11 +2645,11 @@ int spk_net_get_info( spk_net * net, spk_net_info * out )
 		out->dt = net->dt;
 		out->steps = net->steps;
 		out->tile_size = (uint64_t)net->tc.tile;
-		out->num_tiles = (uint64_t)net->tc.ntiles;
+		out->num_tiles = (uint64_t)net->ctas();
 		out->device_bytes = net->device_bytes();
 		out->kernel_launches = net->kernel_launches;
 		out->persistent = net->persistent ? 1 : 0;
-		out->slice_pack = net->flat ? net->pack : 0;
+		out->slice_pack = net->flat ? ( net->dense ? 12 : net->pack ) : 0;
 		out->slot_vecs = net->slot_vecs;
 	} );
 }
@@ -2505,7 +2788,9 @@ int spk_net_restore( spk_net ** out, void const * buf, uint64_t size, int device
 			dir.emplace_back( id, bytes, in );
 			in += bytes;
 		}
-		validate_checkpoint( h, first, dir );
+		double syn = 0, max_in = 0;
+		std::vector<char> in_tile( h.ntiles, 0 );
+		validate_checkpoint( h, first, dir, syn, max_in, in_tile );
 
 		std::unique_ptr<spk_net> net( new_net( h.model, h.dt, h.delay, h.seed, device ) );
 		device_guard g( device );
@@ -2518,6 +2803,9 @@ int spk_net_restore( spk_net ** out, void const * buf, uint64_t size, int device
 		net->flat_tmax = h.flat_tmax;
 		net->tc = { h.threads, h.npt, h.tile, h.ntiles };
 		net->opts.slots = h.slot_vecs; // the saved net's kernel and layout
+		// window_flat's and window_dense's nets are saved alike: the tiling and the graph say
+		// which of the two runs them
+		net->dense = net->flat && h.slot_vecs == 0 && net->opts.bitmaps && dense_fits( h.model, device, h.n, h.delay, syn, max_in, first, in_tile, h.pack );
 		set_tiles( *net, first );
 		net->ring_slots = h.ring_slots;
 		allocate_buffers( *net );
@@ -2545,6 +2833,13 @@ int spk_net_restore( spk_net ** out, void const * buf, uint64_t size, int device
 		for( auto const & x : ckpt_plastic( *net ) )
 			if( x.second->bytes )
 				CK( cudaMemcpyAsync( x.second->p, find( x.first, x.second->bytes ), x.second->bytes, cudaMemcpyHostToDevice, net->stream ) );
+		if( net->dense ) // its step lists, from the restored ring
+			dispatch( net->model, [&]( auto tag ) {
+				using M = typename decltype( tag )::type;
+				if constexpr( spk::is_dense_model<M> )
+					spk::dense_lists_from_ring<M><<<net->delay, 256, 0, net->stream>>>( net->params(), (long long)h.steps );
+			} );
+		CK( cudaGetLastError() );
 		summaries_from_ring( *net ); // slotted nets: the summaries of the restored ring
 		CK( cudaStreamSynchronize( net->stream ) );
 		net->steps = net->launched = h.steps;

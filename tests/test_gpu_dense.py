@@ -1,0 +1,100 @@
+"""window_dense (rows as target bitmaps, the automatic choice for dense nets) against
+window_flat on index lists (slice_bits=16) and, for bursts, against the CPU oracle: persistent
+recording runs, single steps, windows in a batch and restored checkpoints, bit for bit, at the
+edges of its tiles, rounds and lists."""
+import numpy as np
+import pytest
+
+import oracle
+import spice_b200
+from spice_b200 import Layout, Snn
+
+pytestmark = pytest.mark.gpu
+
+B = [(0, 1, 0.1), (1, 1, 0.1)]
+NETS = [
+    # (model, pops, conns, delay, steps): tile edges (255 / 256 / 257 neurons with inputs)
+    ("brunel", [300, 255], B, 15, 331),
+    ("brunel", [300, 256], B, 16, 331),
+    ("brunel", [31, 257], [(0, 1, 0.3), (1, 1, 0.3)], 15, 331),
+    # rounds: five, two and one step, the serial form at delays 1 and 2, runs that end inside a round
+    ("brunel", [1501, 1499], B, 20, 207),
+    ("brunel", [1501, 1499], B, 8, 208),
+    ("brunel", [1501, 1499], B, 3, 209),
+    ("brunel", [1501, 1499], B, 2, 210),
+    ("vogels_abbott", [2999], [(0, 0, 0.05)], 2, 211),
+    # tiles with and without inputs in turn, uneven densities, a population nobody reaches last
+    ("brunel", [997, 401, 1203, 333], [(0, 1, 0.2), (0, 2, 0.05), (2, 1, 0.3), (1, 2, 0.11), (2, 2, 0.04)], 7, 301),
+    # one input class, and the variant of the benchmark configuration
+    ("synth", [5000], [(0, 0, 0.04)], 6, 205),
+    ("brunel_fixed", [2500, 2500], B, 15, 205),
+    # p = 1: the high bytes of the counts
+    ("synth", [70_000], [(0, 0, 0.02)], 5, 60),
+    ("brunel", [20_000, 300], [(0, 1, 1.0)], 15, 120),
+]
+
+
+def bits_equal(a, b):
+    return np.array_equal(np.asarray(a).view(np.uint32), np.asarray(b).view(np.uint32))
+
+
+def same(a, b):
+    for x, y in zip(a.neurons(), b.neurons()):
+        assert bits_equal(x, y)
+
+
+@pytest.mark.parametrize("model,pops,conns,delay,steps", NETS)
+def test_bitmaps_match_slices(model, pops, conns, delay, steps):
+    lay, cap = Layout(pops, conns), sum(pops) * steps
+    a = Snn(model, lay, delay=delay, seed=5, graph_seed=6, options={"kernel": "window"})
+    b = Snn(model, lay, delay=delay, seed=5, graph_seed=6, options={"kernel": "window", "slice_bits": 16})
+    assert a.info().slice_pack == 12 and b.info().slice_pack == 8
+    ca, ia = a.run_record(steps, cap=cap)
+    cb, ib = b.run_record(steps, cap=cap)
+    assert np.array_equal(ca, cb) and np.array_equal(ia, ib)
+    same(a, b)
+    for k in range(2 * delay + 3):  # launches of one step after the persistent one
+        assert np.array_equal(a.step(out=True), b.step(out=True)), k
+    for n in (1, 2, 3, delay + 1):
+        a.run(n)
+        b.run(n)
+    same(a, b)
+    r = Snn.restore(a.checkpoint())
+    r.run(3 * delay + 5)
+    b.run(3 * delay + 5)
+    same(r, b)
+
+
+def test_bitmaps_in_a_batch():
+    """Windows of shared launches, nets of different delays."""
+    specs = [("brunel", [1100, 1300], B, 15), ("brunel", [901, 402], B, 4), ("vogels_abbott", [1400], [(0, 0, 0.06)], 8)]
+    batch = spice_b200.Batch()
+    alone, batched = [], []
+    for i, (model, pops, conns, delay) in enumerate(specs):
+        alone.append(Snn(model, Layout(pops, conns), delay=delay, seed=i, graph_seed=i, options={"slice_bits": 16}))
+        batched.append(Snn(model, Layout(pops, conns), delay=delay, seed=i, graph_seed=i))
+        batch.add(batched[-1])
+    for n in (77, 1, 2, 160):
+        batch.run(n)
+        for a in alone:
+            a.run(n)
+    for a, b in zip(alone, batched):
+        same(a, b)
+    batch.close()
+
+
+@pytest.mark.parametrize("n,delay", [(4000, 8), (9000, 15)])
+def test_bursts_match_the_oracle(n, delay):
+    """VA from rest fires all of its neurons in one step: more arrivals than a step's list in
+    shared memory holds (9,000 at five steps a round), and their echoes."""
+    net = Snn("vogels_abbott", Layout([n], [(0, 0, 0.03)]), delay=delay, seed=1, graph_seed=2)
+    assert net.info().slice_pack == 12
+    edges, width = net.adj()
+    ref = oracle.OracleNet("vogels_abbott", [n], [(0, 0, 0.03)], delay=delay, seed=1, edges=edges, width=width)
+    counts, ids = net.run_record(260, cap=n * 260)
+    o = np.concatenate([[0], np.cumsum(counts)]).astype(int)
+    for k in range(260):
+        assert np.array_equal(ids[o[k]:o[k + 1]], ref.step()), k
+    assert counts.max() == n
+    for x, y in zip(net.neurons(), ref.neurons()):
+        assert bits_equal(x, y)
