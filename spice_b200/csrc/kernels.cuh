@@ -445,14 +445,22 @@ __global__ void __launch_bounds__( 512, 1 ) window_counts( net_params p, int L, 
 }
 
 // ------------------------------------------------------------------------------------
-// graph generation: one warp per row, Bernoulli trials from Philox, warp-scan compaction
-// keeps rows ascending; truncation at `width`; INT_MAX padding with 16-byte stores.
+// graph generation: one warp per row. A lane draws 32 consecutive candidates (eight Philox
+// blocks; what depends on the row only is drawn out of the loop) into a mask; one warp scan
+// per 1,024 candidates places the hits, ascending, in shared memory, from where they are
+// written in whole runs. Truncation at `width`; INT_MAX padding with 16-byte stores. Bound by
+// the generator's multiplications. 4.15 GB of rows (1e10 candidates, p = 0.1) in 8.0 ms; 14.7
+// with one block and one scan per lane and turn of 128 candidates, 0.42 GB in 0.83 instead
+// of 1.52.
 // ------------------------------------------------------------------------------------
+constexpr int GEN_BLOCK = 1024; // candidates of a turn
 __global__ void __launch_bounds__( 256 ) generate_ell( int n, int width, int nconn, conn_dev const * conns, unsigned long long seed, int * edges )
 {
+	__shared__ int hits[8][GEN_BLOCK];
 	int const warp = ( blockIdx.x * blockDim.x + threadIdx.x ) >> 5, lane = threadIdx.x & 31;
 	if( warp >= n ) return;
 	int const src = warp;
+	int * const buf = hits[threadIdx.x >> 5];
 	int * row = edges + (long long)src * width;
 	uint32_t const k0 = (uint32_t)seed, k1 = (uint32_t)( seed >> 32 );
 	int k = 0;
@@ -461,28 +469,33 @@ __global__ void __launch_bounds__( 256 ) generate_ell( int n, int width, int nco
 		conn_dev const c = conns[ci];
 		if( src < c.src_first || src >= c.src_last ) continue;
 		int const range = c.dst_last - c.dst_first;
-		for( int base = 0; base < range && k < width; base += 128 )
+		// every draw is below a threshold of 2^32 (p = 1)
+		bool const all = c.thr > 0xFFFFFFFFull;
+		uint32_t const thr = (uint32_t)c.thr;
+		for( int base = 0; base < range && k < width; base += GEN_BLOCK )
 		{
-			int const j0 = base + 4 * lane;
-			unsigned bits = 0;
+			int const j0 = base + 32 * lane;
+			unsigned bits = 0u;
 			if( j0 < range )
 			{
-				u32x4 const r = philox4x32_10( { (uint32_t)src, (uint32_t)( j0 >> 2 ), (uint32_t)ci, TAG_GRAPH }, k0, k1 );
-				bits = ( (unsigned long long)r.x < c.thr ? 1u : 0u ) | ( ( j0 + 1 < range && (unsigned long long)r.y < c.thr ) ? 2u : 0u ) |
-				       ( ( j0 + 2 < range && (unsigned long long)r.z < c.thr ) ? 4u : 0u ) |
-				       ( ( j0 + 3 < range && (unsigned long long)r.w < c.thr ) ? 8u : 0u );
+#pragma unroll
+				for( int b = 0; b < 8; b++ )
+				{
+					u32x4 const r = philox4x32_10( { (uint32_t)src, (uint32_t)( ( j0 >> 2 ) + b ), (uint32_t)ci, TAG_GRAPH }, k0, k1 );
+					bits |= ( r.x < thr ? 1u << ( 4 * b ) : 0u ) | ( r.y < thr ? 2u << ( 4 * b ) : 0u ) | ( r.z < thr ? 4u << ( 4 * b ) : 0u ) |
+					        ( r.w < thr ? 8u << ( 4 * b ) : 0u );
+				}
+				if( all ) bits = ~0u;
+				if( range - j0 < 32 ) bits &= ( 1u << ( range - j0 ) ) - 1u;
 			}
 			int const cntl = __popc( bits );
-			int const incl = warp_inclusive_scan( cntl );
-			int pos = k + incl - cntl;
-#pragma unroll
-			for( int q = 0; q < 4; q++ )
-				if( ( bits >> q ) & 1u )
-				{
-					if( pos < width ) row[pos] = c.dst_first + j0 + q;
-					pos++;
-				}
-			k = min( width, k + __shfl_sync( 0xffffffffu, incl, 31 ) );
+			int const incl = warp_inclusive_scan( cntl ), total = __shfl_sync( 0xffffffffu, incl, 31 );
+			for( int pos = incl - cntl; bits; bits &= bits - 1u ) buf[pos++] = c.dst_first + j0 + __ffs( bits ) - 1;
+			__syncwarp();
+			int const take = min( total, width - k );
+			for( int e = lane; e < take; e += 32 ) row[k + e] = buf[e];
+			__syncwarp();
+			k += take;
 		}
 	}
 	// padding: scalar up to a 4-aligned position, then int4 stores
