@@ -141,12 +141,13 @@ struct dbuf
 	}
 };
 
-// 16-byte pinned host slots for the nets' small device-to-host reads, carved from slabs
-// allocated once: a page-locked allocation synchronises the whole device, which a net
-// built beside a running batch should not do
+// Pinned host slots for the nets' small device-to-host reads (a step's first spikes among
+// them), carved from slabs allocated once: a page-locked allocation synchronises the whole
+// device, which a net built beside a running batch should not do
 class pinned_slots
 {
 public:
+	static constexpr size_t SLOT = 4096;
 	static unsigned * get()
 	{
 		std::lock_guard<std::mutex> lk( mu() );
@@ -155,7 +156,7 @@ public:
 		{
 			void * slab = nullptr;
 			CK( cudaMallocHost( &slab, SLAB ) );
-			for( size_t o = 0; o < SLAB; o += 16 ) f.push_back( reinterpret_cast<unsigned *>( static_cast<char *>( slab ) + o ) );
+			for( size_t o = 0; o < SLAB; o += SLOT ) f.push_back( reinterpret_cast<unsigned *>( static_cast<char *>( slab ) + o ) );
 		}
 		unsigned * q = f.back();
 		f.pop_back();
@@ -169,7 +170,7 @@ public:
 	}
 
 private:
-	static constexpr size_t SLAB = 64 * 1024;
+	static constexpr size_t SLAB = 64 * SLOT;
 	static std::mutex & mu()
 	{
 		static std::mutex m;
@@ -494,7 +495,7 @@ struct spk_net
 	unsigned long long launched = 0; // steps launched
 	unsigned long long kernel_launches = 0; // simulation kernel launches (graph replays counted per window)
 	int ring_slots = 0;                      // steps the spike ring holds (2 delay; more for recording runs)
-	unsigned * host_count = nullptr; // pinned (a pinned_slots slot)
+	unsigned * host_count = nullptr; // pinned and mapped (a pinned_slots slot)
 
 	cudaGraphExec_t graph = nullptr;
 	int graph_windows = 0, graph_len = 0;
@@ -2513,15 +2514,23 @@ int spk_net_step( spk_net * net, int32_t * out_ids, uint64_t cap, uint64_t * out
 			return;
 		}
 		net->flush();
-		CK( cudaMemsetAsync( net->cursor.p, 0, 8, net->stream ) );
-		net->gather( 1, net->gather_ids.as<int>(), net->gather_cnt.as<unsigned>(), (unsigned long long)net->n, 0 );
-		CK( cudaMemcpyAsync( net->host_count, net->gather_cnt.p, 4, cudaMemcpyDeviceToHost, net->stream ) );
-		net->check_device_error();
-		uint64_t const c = net->host_count[0];
+		// the spikes, their number and the error word straight into the net's pinned slot
+		constexpr int INLINE = (int)pinned_slots::SLOT / 4 - 4;
+		unsigned * const host = net->host_count;
+		spk::gather_step<<<1, 512, 0, net->stream>>>(
+		    net->ring_ids.as<int>(), net->ring_cnt.as<unsigned>(), (int)net->n, net->tile_first.as<int>(), net->tc.ntiles, net->ring_slots,
+		    net->clock.as<spk::clock_state>(), net->err.as<int>(), net->gather_ids.as<int>(), host, INLINE );
+		CK( cudaGetLastError() );
+		CK( cudaStreamSynchronize( net->stream ) );
+		if( host[1] ) throw spk_error( SPK_ERR_DEVICE, "device error flag " + std::to_string( (int)host[1] ) );
+		uint64_t const c = host[0];
 		if( out_count ) *out_count = c;
 		if( !out_ids ) return;
 		if( c > cap ) throw spk_error( SPK_ERR_CAPACITY, "spike buffer too small" );
-		if( c ) CK( cudaMemcpyAsync( out_ids, net->gather_ids.p, c * 4, cudaMemcpyDeviceToHost, net->stream ) );
+		uint64_t const first = std::min<uint64_t>( c, INLINE );
+		std::memcpy( out_ids, host + 4, first * 4 );
+		if( c == first ) return;
+		CK( cudaMemcpyAsync( out_ids + first, net->gather_ids.as<int>() + first, ( c - first ) * 4, cudaMemcpyDeviceToHost, net->stream ) );
 		CK( cudaStreamSynchronize( net->stream ) );
 	} );
 }

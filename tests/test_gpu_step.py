@@ -1,0 +1,41 @@
+"""step(out=True) (gather_step: the spikes written straight to host memory) against recorded
+runs: steps of no spikes, more spikes than its pinned slot holds, more tiles than threads,
+several windows queued before it."""
+import numpy as np
+import pytest
+
+import spice_b200
+from spice_b200 import Layout, Snn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("model,pops,conns,delay,warm,options", [
+    ("vogels_abbott", [3000], [(0, 0, 0.05)], 1, 130, None),          # from rest: none, then all at once
+    ("vogels_abbott", [3000], [(0, 0, 0.05)], 8, 130, {"kernel": "ordered"}),
+    ("synth", [260_000], [(0, 0, 0.00004)], 3, 7, None),              # 1,300 spikes a step
+    ("synth", [700_000], [(0, 0, 0.00001)], 2, 3, {"kernel": "direct"}),
+    ("brunel_with_plasticity", [900, 900], [(0, 1, 0.1), (1, 1, 0.1)], 15, 31, None),
+    ("brunel", [1, 1], [(0, 1, 1.0)], 15, 3, None),
+])
+def test_steps_equal_a_recorded_run(model, pops, conns, delay, warm, options):
+    n, lay = sum(pops), Layout(pops, conns)
+    a = Snn(model, lay, delay=delay, seed=4, graph_seed=4, options=options)
+    b = Snn(model, lay, delay=delay, seed=4, graph_seed=4, options=options)
+    for _ in range(warm):
+        a.step()
+    counts, ids = b.run_record(warm + 25, cap=n * (warm + 25) if n < 10_000 else None)
+    o = np.concatenate([[0], np.cumsum(counts)]).astype(int)
+    for k in range(warm, warm + 25):
+        assert np.array_equal(a.step(out=True), ids[o[k]:o[k + 1]]), k
+
+
+def test_small_buffers_still_report_the_count():
+    import ctypes as C
+
+    net = Snn("synth", Layout(260_000, 0.00004), delay=3, seed=4, graph_seed=4)
+    buf, cnt = np.zeros(100, np.int32), C.c_uint64()
+    lib = spice_b200.library()
+    assert lib.spk_net_step(net._h, buf.ctypes.data, 100, C.byref(cnt)) == spice_b200.ERR_CAPACITY
+    assert cnt.value > 1000 and not buf.any()
+    assert lib.spk_net_step(net._h, None, 0, C.byref(cnt)) == spice_b200.OK and cnt.value > 1000
