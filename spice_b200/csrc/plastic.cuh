@@ -16,6 +16,15 @@
 //     replayed lazily from d's 64-step spike history when the row of s is next touched:
 //     at its next arrival, or at a forced "flush" touch that the owner of s schedules at
 //     most 63 steps after the first pre-active step of the pending window.
+// Between the steps of a window the completion does not walk the rows again: the arrivals'
+// walk already lists the (row, target) pairs whose target will be post-active after the step
+// (its trace decides that, but for its own spike), and the completion takes the list. The
+// first step of a window, whose arrivals an earlier launch walked, steps whose rows are
+// pre-active while a target fired, and lists that overflow take the rows. Once neurons have
+// been silent for long (1,000 steps on), walking every row twice had doubled the step: us
+// per step before and after, 1e6 synapses 13.0 and 9.6, 5e7 22.2 and 18.4, 5e8 50 and 43.5.
+// (Before that, while no target is post-active, the step is 7 to 9 % longer than without
+// lists: 6.85 and 7.35, 41.2 and 44.8; a second walk without them did not change it.)
 // Every touch of row s is announced by the tile that owns neuron s, `delay` steps ahead,
 // through the spike ring (arrivals) or the flush ring, with the trace values the touching
 // tiles need (so no tile reads state another tile writes during the same launch).
@@ -44,6 +53,8 @@ constexpr int PL_THREADS = 384;
 constexpr int PL_CTAS_PER_SM = 2;
 constexpr int PL_STAGE = 256;     // staged arrivals per batch
 constexpr int PL_FLUSH_AT = 63;   // longest replay window (bits of the spike history)
+constexpr int PL_PAST = 64;       // steps before the launch that a replay window may reach
+constexpr int PL_LIST = 2;        // pairs listed for completion, per neuron of the tile
 constexpr int PL_MAX_DELAY = 63;
 
 struct plastic_params
@@ -152,15 +163,16 @@ __device__ __forceinline__ void stage_flushes( net_params const & p, plastic_par
 	}
 }
 
-// Zpre_s over a replay window: zwin[i] = Zpre_s(tp - rf_off + i), no arrivals inside.
-template <typename Syn>
-__device__ __forceinline__ void window_trace( float zrf, int rf_off, long long tp, long long t0, float const * s_dt, float const * dt_ring, float * zwin )
+// Zpre_s over a replay window: zwin[i] = Zpre_s(tp - rf_off + i), no arrivals inside, with the
+// decay factors of its steps dec[i]. The roundings are a chain; the factors come from a table
+// of the launch (s_dec), so that a link is one multiplication.
+__device__ __forceinline__ void window_trace( float zrf, int rf_off, float const * dec, float * zwin )
 {
 	float z = zrf;
+#pragma unroll 8
 	for( int i = 0; i < rf_off; i++ )
 	{
-		long long const tau = tp - rf_off + i;
-		z = fmaf( z, Syn::trace_decay( dt_at( tau, t0, s_dt, dt_ring ) ), 0.0f );
+		z = fmaf( z, dec[i], 0.0f );
 		zwin[i] = z;
 	}
 }
@@ -179,8 +191,13 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 	__shared__ float s_dt[2 * MAX_WINDOW];
 	__shared__ long long s_t0;
 	__shared__ float s_c, s_sum;
-	__shared__ int s_flags; // bit 0: some plastic target post-active at t-1; bit 1: some target fired at t-1
+	__shared__ int s_flags; // bit 0: some plastic target post-active at t-1; bit 1: some target fired at t-1;
+	                        // bit 2: some plastic target will be post-active at t unless it fires
 	__shared__ int s_src[PL_CHUNK];
+	__shared__ float s_dec[PL_PAST + MAX_WINDOW]; // trace decay of step tau at tau - t0 + PL_PAST
+	// step k at k & 1: pairs listed for completion; whether the completion needs the rows all
+	// the same (an arriving row was pre-active, or a target is post-active by its own spike)
+	__shared__ int s_listed[2], s_rows[2];
 
 	int const T = p.tile, tid = threadIdx.x;
 	int const warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
@@ -196,6 +213,8 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 	int * pref = reinterpret_cast<int *>( sh_dpa + ( ( T + 15 ) & ~15 ) );            // [ntiles + 1]
 	stage_e * sb = reinterpret_cast<stage_e *>( pref + ( ( p.ntiles + 1 + 3 ) & ~3 ) ); // [PL_STAGE]
 	float * zwin = reinterpret_cast<float *>( sb + PL_STAGE );                        // [nwarps][64]
+	int4 * list = reinterpret_cast<int4 *>( zwin + nw * 64 );                        // [PL_LIST T] { row, position, target, row's trace }
+	int const list_cap = PL_LIST * T;
 
 	// clock: the window's dt plus `delay` steps of look-ahead for the owners' traces
 	if( tid == 0 )
@@ -213,6 +232,11 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 	}
 	__syncthreads();
 	long long const t0 = s_t0;
+	for( int x = tid; x < PL_PAST + L; x += blockDim.x )
+	{
+		long long const tau = t0 - PL_PAST + x;
+		s_dec[x] = tau >= 0 ? Syn::trace_decay( dt_at( tau, t0, s_dt, p.dt_ring ) ) : 0.0f;
+	}
 
 	// per-neuron state into registers / shared memory
 	Tup st[NPT];
@@ -242,8 +266,10 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 			device_backend bak( p.seed, (uint32_t)i, 0u );
 			bool const dpa = t0 >= 1 && Syn::plastic_dst( (int)i, info ) &&
 			                 Syn::depression_active( zp, p.dt_ring[( t0 - 1 + DT_RING ) % DT_RING], bak );
-			sh_dpa[local] = dpa;
-			any_pa |= dpa;
+			// bit 0: post-active after step t - 1; bit 1: after step t, unless it fires in it
+			bool const next = Syn::plastic_dst( (int)i, info ) && Syn::depression_active( fmaf( zp, Syn::trace_decay( s_dt[0] ), 0.0f ), s_dt[0], bak );
+			sh_dpa[local] = ( dpa ? 1 : 0 ) | ( next ? 2 : 0 );
+			any_pa |= ( dpa ? 1 : 0 ) | ( next ? 4 : 0 );
 			any_fired |= (int)( h & 1ull );
 		}
 		else if( local < T )
@@ -254,9 +280,14 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 		}
 	}
 	for( int x = tid; x < T; x += blockDim.x ) mask[x] = 0;
-	if( tid == 0 ) s_flags = 0;
+	if( tid == 0 )
+	{
+		s_flags = 0;
+		s_listed[0] = s_listed[1] = 0;
+		s_rows[0] = s_rows[1] = 0;
+	}
 	__syncthreads();
-	if( any_pa ) atomicOr( &s_flags, 1 );
+	if( any_pa ) atomicOr( &s_flags, any_pa );
 	if( any_fired ) atomicOr( &s_flags, 2 );
 	__syncthreads();
 
@@ -269,14 +300,34 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 		if( t - 1 >= p.delay )
 		{
 			int const slot_c = (int)( ( t - 1 - p.delay ) % p.ring );
+			// uniform: written before the last step's barriers
+			int const count = s_listed[( k + 1 ) & 1];
+			bool const listed = k > 0 && count <= list_cap && !( s_rows[( k + 1 ) & 1] && ( s_flags & 2 ) );
 			bool pot_any = false;
-			if( s_flags & 2 )
+			if( !listed && ( s_flags & 2 ) )
 				for( int i = lane; i < p.ntiles; i += 32 ) pot_any |= q.ring_pot[(long long)slot_c * p.ntiles + i] != 0;
 			pot_any = __any_sync( 0xffffffffu, pot_any );
 			bool const need = ( s_flags & 1 ) || ( ( s_flags & 2 ) && pot_any );
 			// `need` may differ between warps only through pot_any, which every warp computed
 			// from the same data: uniform.
-			if( need )
+			if( listed )
+			{
+				if( need )
+				{
+					float const dt_c = s_dt[k - 1];
+					for( int x = tid; x < count; x += blockDim.x )
+					{
+						int4 const e = list[x];
+						if( !( sh_dpa[e.z] & 1 ) ) continue;
+						float * const wp = q.W + (long long)e.x * p.width + e.y;
+						device_backend bak( p.seed, (uint32_t)e.x, (uint32_t)t );
+						float const w = *wp;
+						float const w2 = Syn::update( w, true, sh_hist[e.z] & 1ull, __int_as_float( e.w ), sh_zpost[e.z], dt_c, bak );
+						if( __float_as_int( w2 ) != __float_as_int( w ) ) *wp = w2;
+					}
+				}
+			}
+			else if( need )
 			{
 				float const dt_c = dt_at( t - 1, t0, s_dt, p.dt_ring );
 				int const total = stage_prefix( p, p.ring_cnt, slot_c, pref, scratch );
@@ -299,7 +350,7 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 							int const local = d - d0;
 							if( (unsigned)local >= (unsigned)span || !Syn::plastic_dst( d, info ) ) continue;
 							bool const x_d = sh_hist[local] & 1ull;
-							if( !sh_dpa[local] && !( x_d && pot ) ) continue;
+							if( !( sh_dpa[local] & 1 ) && !( x_d && pot ) ) continue;
 							float const w = wrow[j];
 							float const w2 = Syn::update( w, true, x_d, e.zt, sh_zpost[local], dt_c, bak );
 							if( __float_as_int( w2 ) != __float_as_int( w ) ) wrow[j] = w2;
@@ -325,7 +376,7 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 					stage_e const e = sb[x];
 					int const rf_off = e.meta & 0xff;
 					float * zw = zwin + warp * 64;
-					if( lane == 0 ) window_trace<Syn>( e.zrf, rf_off, t, t0, s_dt, p.dt_ring, zw );
+					if( lane == 0 ) window_trace( e.zrf, rf_off, s_dec + ( t - rf_off - t0 + PL_PAST ), zw );
 					__syncwarp();
 					int const * row = p.edges + (long long)e.src * p.width;
 					float * wrow = q.W + (long long)e.src * p.width;
@@ -407,11 +458,12 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 					auto arrive = [&]( int x, bool ahead1st, int d1st, float w1st, int d2nd, float w2nd ) {
 						stage_e const e = sb[c0 + x];
 						int const rf_off = e.meta & 0xff;
-						bool const replay = rf_off > 0 && Syn::plastic_src( e.src, info );
+						bool const plastic = Syn::plastic_src( e.src, info ), replay = rf_off > 0 && plastic, listing = plastic && ( s_flags & 4 );
+						if( plastic && ( e.meta >> 8 & 1 ) && lane == 0 ) s_rows[k & 1] = 1;
 						float * zw = zwin + warp * 64;
 						if( replay )
 						{
-							if( lane == 0 ) window_trace<Syn>( e.zrf, rf_off, t, t0, s_dt, p.dt_ring, zw );
+							if( lane == 0 ) window_trace( e.zrf, rf_off, s_dec + ( t - rf_off - t0 + PL_PAST ), zw );
 							__syncwarp();
 						}
 						int const * row = p.edges + (long long)e.src * p.width;
@@ -444,6 +496,11 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 							}
 							wcol[local] = w;
 							atomicOr( mask + local, bit );
+							if( listing && ( sh_dpa[local] & 2 ) )
+							{
+								int const o = atomicAdd( &s_listed[k & 1], 1 );
+								if( o < list_cap ) list[o] = make_int4( e.src, j, local, __float_as_int( e.zt ) );
+							}
 						}
 						if( replay ) __syncwarp();
 					};
@@ -511,6 +568,7 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 		bool pot_tile = false;
 		int apa = 0, afi = 0;
 		float const c_t = Syn::trace_decay( dt_t );
+		float const dt_next = s_dt[k + 1], c_next = Syn::trace_decay( dt_next );
 		long long const ta = t + p.delay; // look-ahead touch step
 		float const dt_a = s_dt[k + p.delay];
 		float const c_a = Syn::trace_decay( dt_a );
@@ -528,11 +586,15 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 				bool const x = N::update( it, dt_t, info, bak );
 				unsigned long long const h = ( sh_hist[local] << 1 ) | ( x ? 1ull : 0ull );
 				float const zp = fmaf( sh_zpost[local], c_t, x ? 1.0f : 0.0f );
-				bool const dpa = Syn::plastic_dst( (int)i, info ) && Syn::depression_active( zp, dt_t, bak );
+				bool const pdst = Syn::plastic_dst( (int)i, info );
+				int const was = sh_dpa[local];
+				bool const dpa = x ? pdst && Syn::depression_active( zp, dt_t, bak ) : ( was & 2 ) != 0;
+				if( x && dpa && !( was & 2 ) ) s_rows[k & 1] = 1; // its pairs were not listed
 				sh_hist[local] = h;
 				sh_zpost[local] = zp;
-				sh_dpa[local] = dpa;
-				apa |= dpa;
+				bool const next = pdst && Syn::depression_active( fmaf( zp, c_next, 0.0f ), dt_next, bak );
+				sh_dpa[local] = ( dpa ? 1 : 0 ) | ( next ? 2 : 0 );
+				apa |= ( dpa ? 1 : 0 ) | ( next ? 4 : 0 );
 				afi |= x;
 				if( x ) fired |= 1u << kk;
 
@@ -571,10 +633,16 @@ __device__ __forceinline__ void window_plastic_body( net_params const & p, plast
 				}
 			}
 		}
-		if( tid == 0 ) s_flags = 0;
+		if( tid == 0 )
+		{
+			s_flags = 0;
+			// the next step's list, last read in this step's completion
+			s_listed[( k + 1 ) & 1] = 0;
+			s_rows[( k + 1 ) & 1] = 0;
+		}
 		int total;
 		int off = block_exclusive_scan( __popc( fired ), scratch, &total ); // syncs: s_flags reset visible
-		if( apa ) atomicOr( &s_flags, 1 );
+		if( apa ) atomicOr( &s_flags, apa );
 		if( afi ) atomicOr( &s_flags, 2 );
 		int const slot_out = (int)( t % p.ring );
 		long long const seg = (long long)slot_out * p.n + d0;
@@ -802,6 +870,7 @@ inline int plastic_window_smem( int tile, int ntiles, int threads )
 	b += (size_t)( ( ntiles + 1 + 3 ) & ~3 ) * 4;
 	b += (size_t)PL_STAGE * sizeof( stage_e );
 	b += (size_t)( threads / 32 ) * 64 * 4;
+	b += (size_t)PL_LIST * tile * 16;
 	return (int)b;
 }
 
