@@ -431,6 +431,10 @@ __device__ __noinline__ void dense_publish( int r, int s )
 	unsigned long long at = 0;
 	if( lane == 0 )
 	{
+		// read before the addition: once the step is complete, a scout of this CTA may move the
+		// word on to the next step of the list's place (in this very tick, where 3 m = delay)
+		unsigned long long const before = *const_cast<unsigned long long volatile *>( dense_at<unsigned long long>( x.words_before ) + l );
+		asm volatile( "" ::"l"( before ) : "memory" );
 		unsigned long long add = 0;
 #pragma unroll
 		for( int h = 0; h < 2; h++ )
@@ -439,7 +443,7 @@ __device__ __noinline__ void dense_publish( int r, int s )
 				x.p.ring_cnt[row * x.p.ntiles + x.tile[h]] = (unsigned)all[h];
 				if( x.tile[h] != x.p.withhold_tile ) add += dense_word( all[h] - one[h], one[h] );
 			}
-		at = atomicAdd( x.p.step_word + l, add ) - dense_at<unsigned long long>( x.words_before )[l];
+		at = atomicAdd( x.p.step_word + l, add ) - before;
 	}
 	int b0 = __shfl_sync( 0xffffffffu, (int)( at & 0xFFFFFF ), 0 ), b1 = __shfl_sync( 0xffffffffu, (int)( at >> 24 & 0xFFFFFF ), 0 );
 #pragma unroll
