@@ -174,7 +174,7 @@ def profile_traffic(syn):
     at (1e9 synapses) only."""
     if syn != 1e9:
         return None
-    path = os.path.join(ROOT, "profiles", "window_flat_brunel_1e9.json")
+    path = os.path.join(ROOT, "profiles", "window_dense_brunel_1e9.json")
     try:
         with open(path) as f:
             d = json.load(f)
@@ -369,7 +369,7 @@ def run_ours(args, rank, world):
                 "sim_steps_per_bench_step": S, "spikes_per_step": spikes_per_step, "setup_s": setup_s,
                 "tiles": info.num_tiles, "tile_size": info.tile_size,
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                             "traffic": traffic, "peak_kind": peak_kind, "kernel": "window_flat<brunel>",
+                             "traffic": traffic, "peak_kind": peak_kind, "kernel": "window_dense<brunel>",
                              "bytes_per_launch": bytes_per_launch, "launch_us": t_launch * 1e6,
                              "steps_per_launch": steps_per_launch, "persistent": persistent,
                              "bytes_per_step": bytes_per_step},

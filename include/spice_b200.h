@@ -69,14 +69,16 @@ typedef struct spk_net_info
 	int delay;             /* snn::delay()  (spice/snn.h:27)                             */
 	float dt;              /* snn::dt()     (spice/snn.h:26)                             */
 	uint64_t steps;        /* steps taken so far                                         */
-	uint64_t tile_size;    /* destination neurons per tile (one CTA each)                */
-	uint64_t num_tiles;
+	uint64_t tile_size;    /* destination neurons per tile at most                       */
+	uint64_t num_tiles;    /* CTAs of a window launch: one per tile (nets on target bitmaps:
+	                          one per pair of tiles, with inputs and without)           */
 	uint64_t device_bytes; /* device memory held by the net                              */
 	uint64_t kernel_launches; /* simulation kernel launches so far (a CUDA graph's replay
 	                             counts each window; a batch counts its shared launches)  */
 	int persistent;        /* 1: spk_net_run advances the net in one cooperative launch */
 	int slice_pack;        /* window_flat slices: 8 (16-bit) or 12 (10-bit) indices per
-	                          16-byte vector; 0 for the other window kernels            */
+	                          16-byte vector; 12 too for nets on target bitmaps
+	                          (window_dense); 0 for the other window kernels            */
 	int slot_vecs;         /* window_slots: 16-byte vectors per fixed (source, tile) slot;
 	                          0 when the net keeps variable slices                     */
 } spk_net_info;
